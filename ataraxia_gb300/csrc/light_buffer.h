@@ -11,24 +11,20 @@
 
 namespace atx {
 
-// Device bytes lb_build needs for nl lights at res cells along a face's edge.
+// Device bytes cells_build needs for the light buffer of nl lights, and for
+// the direction buffer of n spheres, at res cells along a face's edge.
 uint64_t lb_bytes(uint32_t nl, uint32_t res);
-
-// Builds the light buffer of the n spheres sph (cx, cy, cz, r*r) with radii
-// radius[] and the nl lights (1 <= nl <= kLbMaxLights, n <= kLbMaxSpheres),
-// res cells along a face's edge (kCellResMin..kCellResMax), into buf
-// (lb_bytes(nl, res) bytes of device memory) on stream; *out views buf.
-cudaError_t lb_build(const float4* sph, const float* radius, uint32_t n, const DevLight* lights, uint32_t nl,
-                     uint32_t res, void* buf, uint64_t bytes, LightBufferView* out, cudaStream_t stream);
-
-// Device bytes db_build needs for n spheres at res cells along a face's edge.
 uint64_t db_bytes(uint32_t n, uint32_t res);
 
-// Builds the direction buffer of the n spheres sph (cx, cy, cz, r*r) with
-// radii radius[] (1 <= n <= kDbMaxSpheres), res cells along a face's edge,
-// into buf (db_bytes(n, res) bytes of device memory) on stream; *out views
-// buf.
-cudaError_t db_build(const float4* sph, const float* radius, uint32_t n, uint32_t res, void* buf, uint64_t bytes,
-                     DirBufferView* out, cudaStream_t stream);
+// Builds, on stream, for the n spheres sph (cx, cy, cz, r*r) with radii
+// radius[], at res cells along a face's edge (kCellResMin..kCellResMax):
+//   the light buffer of the nl lights (1 <= nl <= kLbMaxLights, n <=
+//   kLbMaxSpheres) into lbuf (lb_bytes(nl, res) bytes of device memory; null:
+//   none), *lv its view;
+//   the direction buffer (n <= kDbMaxSpheres) into dbuf (db_bytes(n, res)
+//   bytes; null: none), *dv its view.
+cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, const DevLight* lights, uint32_t nl,
+                        uint32_t res, void* lbuf, uint64_t lbytes, LightBufferView* lv, void* dbuf, uint64_t dbytes,
+                        DirBufferView* dv, cudaStream_t stream);
 
 }  // namespace atx

@@ -108,27 +108,22 @@ atx_status SceneStore::build_cells(Budget* budget, cudaStream_t stream)
 {
     const uint32_t n = view.n_sph, nl = view.n_lights;
     const uint32_t res = cell_res ? cell_res : default_cell_res(n);
-    // light buffer for the shadow rays of the brute-force tables
+    // light buffer for the shadow rays of the brute-force tables, direction
+    // buffer for their extension rays
+    const bool lb = !view.use_bvh && n >= 1 && n <= kLbMaxSpheres && nl >= 1 && nl <= kLbMaxLights;
+    const bool db = !view.use_bvh && n >= 1 && n <= kDbMaxSpheres;
     view.lb = LightBufferView{};
-    if (!view.use_bvh && n >= 1 && n <= kLbMaxSpheres && nl >= 1 && nl <= kLbMaxLights) {
-        ATX_TRY(lbuf.ensure(lb_bytes(nl, res), budget, "light buffer"));
-        LightBufferView lv{};
-        ATX_CUDA(lb_build(view.sph, sph_rad.as<float>(), n, view.lights, nl, res, lbuf.get(), lbuf.bytes(), &lv,
-                          stream));
-        view.lb = lv;
-    } else {
-        lbuf.reset();
-    }
-    // direction buffer for the extension rays of the brute-force tables
     view.db = DirBufferView{};
-    if (!view.use_bvh && n >= 1 && n <= kDbMaxSpheres) {
-        ATX_TRY(dbuf.ensure(db_bytes(n, res), budget, "direction buffer"));
-        DirBufferView dv{};
-        ATX_CUDA(db_build(view.sph, sph_rad.as<float>(), n, res, dbuf.get(), dbuf.bytes(), &dv, stream));
-        view.db = dv;
-    } else {
-        dbuf.reset();
-    }
+    if (!lb) lbuf.reset();
+    if (!db) dbuf.reset();
+    if (lb) ATX_TRY(lbuf.ensure(lb_bytes(nl, res), budget, "light buffer"));
+    if (db) ATX_TRY(dbuf.ensure(db_bytes(n, res), budget, "direction buffer"));
+    LightBufferView lv{};
+    DirBufferView dv{};
+    ATX_CUDA(cells_build(view.sph, sph_rad.as<float>(), n, view.lights, nl, res, lb ? lbuf.get() : nullptr,
+                         lbuf.bytes(), &lv, db ? dbuf.get() : nullptr, dbuf.bytes(), &dv, stream));
+    view.lb = lv;
+    view.db = dv;
     return ATX_OK;
 }
 
