@@ -301,10 +301,9 @@ atx_status enqueue_frames(const SceneView& sc, const CameraView& cam, WaveStore&
             // (in the cache, or in the wave's own per-pixel rows, which only k_primary writes)
             job.prim_cached = filled ? 1 : 0;
             ATX_CUDA(enqueue_wave(sc, cam, ws.view, job, shape, accum, image, stream, launches, timer));
-            if (wave_shares_primary(job)) filled = true;
-            // primary rays traced: once per pixel when its samples share the hit, none when cached
-            if (primary_rays && max_bounces > 0 && !job.prim_cached)
-                *primary_rays += wave_shares_primary(job) ? np : (uint64_t)np * job.spp;
+            if (max_bounces > 0) filled = true;
+            // primary rays traced: once per pixel (its samples share the hit), none when cached
+            if (primary_rays && max_bounces > 0 && !job.prim_cached) *primary_rays += np;
         }
     }
     return ATX_OK;

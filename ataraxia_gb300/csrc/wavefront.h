@@ -199,10 +199,8 @@ struct WaveState {
 constexpr uint64_t kWaveBytesPerPath = 7 * 16 + 4 * 4 + 8;
 constexpr uint64_t kWaveArrays = 12;
 
-// Counter slots after the per-bounce pairs: [2*(max_bounces+1)] = hit pixels,
-// [2*(max_bounces+1)+1] = paths shaded at the first bounce (counted only when
-// the wave does not share primary hits; else it is hit pixels x spp),
-// [2*(max_bounces+1)+2] = rays of k_paths' starting queue claimed so far,
+// Counter slots after the per-bounce pairs: [2*(max_bounces+1)] = hit pixels
+// (the next one is unused), [2*(max_bounces+1)+2] = rays of k_paths' starting queue claimed so far,
 // [2*(max_bounces+1)+3] = extension rays traced that no queue counts (with a
 // light buffer a ray is traced where it is made and only hits are queued:
 // the misses, and every ray k_paths traces).
@@ -227,23 +225,17 @@ struct WaveJob {
     int32_t prim_cached;
 };
 
-// Whether a wave shares each pixel's primary hit among its samples (the hit is
-// traced once, by k_primary, or comes from the cache).
-__host__ __device__ inline bool wave_shares_primary(const WaveJob& j)
-{
-    return j.max_bounces > 0 && (j.spp > 1 || j.prim_cache != nullptr);
-}
-
 // Whether the first bounce's shadow rays are traced once per (pixel, light)
 // instead of once per sample.  A pixel's samples share the primary hit, so
 // samples that pick the same light (Renderer.cu:339, PcgHash(seed) % lights)
 // cast the same shadow ray: k_primary queues one ray per distinct light the
 // pixel's samples pick, k_shadow records the visible ones in ws.vis, and the
-// first bounce adds the light of a sample whose light is visible.  Needs the
-// light set to fit one 32-bit word (and a wave's hit slots 26 bits).
+// first bounce adds the light of a sample whose light is visible.  Needs
+// several samples per pixel (one sample picks one light), and the light set to
+// fit one 32-bit word (and a wave's hit slots 26 bits).
 __host__ __device__ inline bool wave_light_vis(const WaveJob& j, uint32_t n_lights)
 {
-    return wave_shares_primary(j) && n_lights > 0u && n_lights <= 32u && j.n_pixels <= (1u << 26);
+    return j.max_bounces > 0 && j.spp > 1u && n_lights > 0u && n_lights <= 32u && j.n_pixels <= (1u << 26);
 }
 
 // Kernel families timed by KernelTimer.
