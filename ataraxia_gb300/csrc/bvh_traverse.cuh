@@ -244,9 +244,10 @@ __device__ __forceinline__ int32_t bvh_nearest(const SceneView& sc, float3 o, fl
 // 32 entries at a time, one per lane, and hands each sphere to every lane by
 // shuffle; the brute-force filter (leaf_candidates' arithmetic) and the exact
 // test decide, and ties go to the lowest original index as in leaf_nearest,
-// so the list's order does not matter.  All 32 lanes call it.
-__device__ __forceinline__ int32_t nearest_listed(const BvhView& b, const uint32_t* __restrict__ list, uint32_t len,
-                                                  float3 o, float3 d, bool me, float& tmin)
+// so the list's order does not matter.  The list lies in global or shared
+// memory.  All 32 lanes call it.
+__device__ __forceinline__ int32_t nearest_listed(const BvhView& b, const uint32_t* list, uint32_t len, float3 o,
+                                                  float3 d, bool me, float& tmin)
 {
     const float a = dot3(d, d);
     const uint32_t lane = threadIdx.x & 31u;
@@ -254,7 +255,7 @@ __device__ __forceinline__ int32_t nearest_listed(const BvhView& b, const uint32
     int32_t best = -1;
     for (uint32_t base = 0; base < len; base += 32u) {
         const uint32_t k = base + lane;
-        const uint32_t s = k < len ? __ldg(&list[k]) : 0u;
+        const uint32_t s = k < len ? list[k] : 0u;
         const float4 v = __ldg(&b.leaf_sph[s]);
         const uint32_t m = min(32u, len - base);
         for (uint32_t j = 0; j < m; ++j) {

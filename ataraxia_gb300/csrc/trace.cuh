@@ -210,9 +210,7 @@ __device__ __forceinline__ bool occluded_brute(const float4* __restrict__ sph, u
 // ------------------------------------------------------------- warp cones
 //
 // Rays of one warp that leave one apex in a narrow cone of directions: the
-// primary rays of 32 neighbouring pixels (apex: the camera), and the
-// first-bounce shadow rays of neighbouring hit points towards one light, seen
-// from the light.  The warp tests every sphere once against the cone of its
+// primary rays of 32 neighbouring pixels (apex: the camera).  The warp tests every sphere once against the cone of its
 // active lanes' directions and the lanes run the exact test only on the
 // spheres that pass, in index order; results equal the brute-force loop's.
 //
@@ -256,6 +254,23 @@ __device__ __forceinline__ bool warp_cone(bool me, float3 w, WarpCone& c)
     return true;
 }
 
+// A warp's 32 consecutive pixels lie in one image row, or at the end of one
+// and the start of the next (and more rows of an image narrower than 32): the
+// lanes of the first row and the others then get a cone each, one after the
+// other.  One cone around both ends of a row is as wide as the image and meets
+// most spheres: with 1279 pixels to a row one warp in 40 tested all of 1,000
+// spheres and its launch waited for it (k_primary with the camera's masks
+// 186 -> 28 us).  Returns how many groups there are and sets first for the
+// lanes of the first.  All 32 lanes call it, lane 0 inside the image; p: the
+// lane's pixel.
+__device__ __forceinline__ uint32_t row_groups(bool me, uint32_t p, uint32_t width, bool& first)
+{
+    const uint32_t row = p / width;
+    const uint32_t row0 = __shfl_sync(0xffffffffu, row, 0);   // by every lane, not behind me
+    first = row == row0;
+    return __any_sync(0xffffffffu, me && !first) ? 2u : 1u;
+}
+
 // Whether a sphere (centre at v from the apex, radius r) may be hit by a ray
 // of the cone.  extra: added to |v| for the origin-to-centre distance D of the
 // margin; e: absolute inflation.  Approximate reciprocal square roots (a few
@@ -284,9 +299,8 @@ __device__ __forceinline__ float cone_radius(float r2)
 
 // Nearest hit of the rays (o, d) of the lanes with me set, all leaving the
 // apex o (the same on every lane) inside cone c.  All 32 lanes call it.
-template <bool SMEM>
-__device__ __forceinline__ int32_t nearest_cone(const float4* __restrict__ sph, uint32_t n, float3 o, float3 d, bool me,
-                                                const WarpCone& c, float& tmin)
+__device__ __forceinline__ int32_t nearest_cone(const float4* __restrict__ sph, uint32_t n, float3 o, float3 d,
+                                                bool me, const WarpCone& c, float& tmin)
 {
     const float a = dot3(d, d);
     const uint32_t lane = threadIdx.x & 31u;
@@ -295,7 +309,7 @@ __device__ __forceinline__ int32_t nearest_cone(const float4* __restrict__ sph, 
     for (uint32_t base = 0; base < n; base += 32u) {
         bool pass = false;
         if (base + lane < n) {
-            const float4 s = table_sphere<SMEM>(sph, base + lane);
+            const float4 s = __ldg(&sph[base + lane]);
             pass = cone_meets(c, mk3(s.x - o.x, s.y - o.y, s.z - o.z), cone_radius(s.w), 0.0f, 0.0f);
         }
         uint32_t mask = __ballot_sync(0xffffffffu, pass);
@@ -303,7 +317,7 @@ __device__ __forceinline__ int32_t nearest_cone(const float4* __restrict__ sph, 
             const uint32_t i = base + (uint32_t)(__ffs(mask) - 1);
             mask &= mask - 1u;
             float t;
-            if (me && sphere_t(table_sphere<SMEM>(sph, i), o, d, a, t) && t > 0.0f && t < tm) {
+            if (me && sphere_t(__ldg(&sph[i]), o, d, a, t) && t > 0.0f && t < tm) {
                 tm = t;
                 best = (int32_t)i;
             }
@@ -313,24 +327,30 @@ __device__ __forceinline__ int32_t nearest_cone(const float4* __restrict__ sph, 
     return best;
 }
 
-// nearest_cone with the candidates read from a tile mask row (words words,
-// bit i % 32 of word i / 32 for sphere i) built with the same cone test for
-// a cone that contains every lane's direction: the same candidates or more,
-// each decided by the same exact test in the same index order.
-template <bool SMEM>
+// nearest_cone with the candidates read from a tile mask row (words <= 32
+// words, bit i % 32 of word i / 32 for sphere i) built with the same cone test
+// for a cone that contains every lane's direction: the same candidates or
+// more, each decided by the same exact test in the same index order.  Lane w
+// loads word w, so the row arrives in one load, and only words with a
+// candidate are looked at.
 __device__ __forceinline__ int32_t nearest_masked(const float4* __restrict__ sph, const uint32_t* __restrict__ row,
                                                   uint32_t words, float3 o, float3 d, bool me, float& tmin)
 {
     const float a = dot3(d, d);
+    const uint32_t lane = threadIdx.x & 31u;
     int32_t best = -1;
     float tm = kFltMax;
-    for (uint32_t w = 0; w < words; ++w) {
-        uint32_t mask = __ldg(&row[w]);
-        while (mask) {   // lowest index first: ties keep it, as in the brute-force loop
-            const uint32_t i = 32u * w + (uint32_t)(__ffs(mask) - 1);
+    const uint32_t mine = lane < words ? __ldg(&row[lane]) : 0u;
+    uint32_t some = __ballot_sync(0xffffffffu, mine != 0u);
+    while (some) {   // lowest index first: ties keep it, as in the brute-force loop
+        const int w = __ffs(some) - 1;
+        some &= some - 1u;
+        uint32_t mask = __shfl_sync(0xffffffffu, mine, w);
+        while (mask) {
+            const uint32_t i = 32u * (uint32_t)w + (uint32_t)(__ffs(mask) - 1);
             mask &= mask - 1u;
             float t;
-            if (me && sphere_t(table_sphere<SMEM>(sph, i), o, d, a, t) && t > 0.0f && t < tm) {
+            if (me && sphere_t(__ldg(&sph[i]), o, d, a, t) && t > 0.0f && t < tm) {
                 tm = t;
                 best = (int32_t)i;
             }
@@ -340,36 +360,82 @@ __device__ __forceinline__ int32_t nearest_masked(const float4* __restrict__ sph
     return best;
 }
 
-// Any hit for the shadow rays (o, d, dist2) of the lanes with me set, whose
-// segments end near the light at apex; c is the cone of the directions from
-// the apex to the origins and dmax the largest apex-to-origin distance.  All
-// 32 lanes call it.
-template <bool SMEM>
-__device__ __forceinline__ bool occluded_cone(const float4* __restrict__ sph, uint32_t n, float3 o, float3 d,
-                                              float dist2, bool me, float3 apex, const WarpCone& c, float dmax)
+// The part of cone_meets that does not depend on the cone, for a sphere seen
+// from the apex of many cones: cone_meets passes it when
+// dot(v, u) >= cos_lo * a - sin_hi * b - e, with a = |v| (1 - sb^2),
+// b = |v| sb, e = 1e-5 |v|; a = -inf: it meets every cone.  Regrouped, the
+// three products differ from cone_meets' by a few 2^-24 |v|, within its 1e-5
+// slack.
+struct ConeCap {
+    float3 v;
+    float a, b, e;
+};
+
+__device__ __forceinline__ ConeCap cone_cap(float4 s, float3 apex)
+{
+    ConeCap c;
+    c.v = mk3(s.x - apex.x, s.y - apex.y, s.z - apex.z);
+    const float d2 = dot3(c.v, c.v);
+    const float inv = rsqrtf(d2);
+    const float dist = d2 * inv;
+    const float m = kBvhK * (dist + 1e-3f);
+    const float R = cone_radius(s.w) * 1.00001f + m;
+    if (!(dist > R + m)) {
+        c.a = __int_as_float(0xff800000);
+        c.b = 0.0f;
+        c.e = 0.0f;
+    } else {
+        const float sb = R * inv * 1.0001f;
+        c.a = dist * (1.0f - sb * sb);
+        c.b = dist * sb;
+        c.e = dist * 1e-5f;
+    }
+    return c;
+}
+
+// Works out the caps of the n spheres seen from the apex into shared memory
+// (cap[i]: v, a; cap2[i]: b, e).  The whole block calls it.
+__device__ __forceinline__ void stage_caps(const float4* __restrict__ sph, uint32_t n, float3 apex, float4* cap,
+                                           float2* cap2)
+{
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const ConeCap c = cone_cap(__ldg(&sph[i]), apex);
+        cap[i] = make_float4(c.v.x, c.v.y, c.v.z, c.a);
+        cap2[i] = make_float2(c.b, c.e);
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ bool cap_in_cone(float4 p, float2 q, const WarpCone& c)
+{
+    return dot3(mk3(p.x, p.y, p.z), c.u) >= c.cos_lo * p.w - c.sin_hi * q.x - q.y;
+}
+
+// nearest_cone over staged caps.
+__device__ __forceinline__ int32_t nearest_caps(const float4* __restrict__ sph, uint32_t n, const float4* cap,
+                                                const float2* cap2, float3 o, float3 d, bool me, const WarpCone& c,
+                                                float& tmin)
 {
     const float a = dot3(d, d);
     const uint32_t lane = threadIdx.x & 31u;
-    bool occ = false;
+    int32_t best = -1;
+    float tm = kFltMax;
     for (uint32_t base = 0; base < n; base += 32u) {
         bool pass = false;
-        if (base + lane < n) {
-            const float4 s = table_sphere<SMEM>(sph, base + lane);
-            // D <= |c - apex| + dmax; the segment's bend (1e-4 offset, float
-            // error of the direction) stays within 2e-4 + kBvhK dmax
-            pass = cone_meets(c, mk3(s.x - apex.x, s.y - apex.y, s.z - apex.z), cone_radius(s.w), 2.0f * dmax, 2e-4f);
-        }
+        if (base + lane < n) pass = cap_in_cone(cap[base + lane], cap2[base + lane], c);
         uint32_t mask = __ballot_sync(0xffffffffu, pass);
-        while (mask) {
+        while (mask) {   // lowest index first: ties keep it, as in the brute-force loop
             const uint32_t i = base + (uint32_t)(__ffs(mask) - 1);
             mask &= mask - 1u;
             float t;
-            if (me && !occ && sphere_t(table_sphere<SMEM>(sph, i), o, d, a, t) && t > 0.0f && t * t < dist2)
-                occ = true;
+            if (me && sphere_t(__ldg(&sph[i]), o, d, a, t) && t > 0.0f && t < tm) {
+                tm = t;
+                best = (int32_t)i;
+            }
         }
-        if (__all_sync(0xffffffffu, occ || !me)) break;
     }
-    return occ;
+    tmin = tm;
+    return best;
 }
 
 // ------------------------------------------------------------ light buffer

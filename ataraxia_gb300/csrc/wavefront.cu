@@ -114,26 +114,122 @@ __device__ __forceinline__ float4 light_dir(const SceneView& sc, uint32_t li, fl
     return l1;
 }
 
+// Candidate spheres of one cone of an LBVH scene: a warp-cooperative walk of
+// the 4-wide nodes (lbvh.cu k_pack_quads).  A slot is entered when the cone
+// meets the ball around its box centre through the box corners, that radius
+// also added to the distance in the float-error margin: this ball, inflated by
+// cone_meets, contains the inflated test ball of every sphere inside the box,
+// so a slot holding a sphere that passes the sphere test is entered.  Eight
+// nodes are popped at a time and their 32 slots tested one per lane (a node a
+// step left 28 lanes idle, and a warp's walk a chain of every node it visits:
+// the lists of a 3840x2160 view of 65,536 spheres took 1,230 + 1,070 us, now
+// 450 + 350); a leaf cluster's spheres get the sphere test the brute-force masks
+// use, one per lane, two clusters of up to 16 at once.  All lanes call it with
+// the warp's own stack in shared memory.  Adds the candidates to the count of
+// those found before (the first cap of them written to out when FILL) and
+// returns it, or kNoTileList when the walk overflows its stack or step budget
+// or the list would pass kTileListMax.
+constexpr uint32_t kWalkStack = 128;
+
+template <bool FILL>
+__device__ uint32_t tile_walk(const BvhView& b, const WarpCone& cone, float3 o, uint32_t* stack, uint32_t count,
+                              uint32_t* out, uint32_t cap)
+{
+    const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
+    uint32_t sp = 1u;
+    uint32_t budget = 2u * b.n_leaves + 8u;
+    __syncwarp();
+    if (lane == 0u) stack[0] = b.root;
+    __syncwarp();
+    while (sp > 0u) {
+        const uint32_t m = min(sp, 8u);
+        if (budget < m) return kNoTileList;
+        budget -= m;
+        const uint32_t node = (lane >> 2) < m ? stack[sp - 1u - (lane >> 2)] : ~0u;
+        sp -= m;
+        bool pass = false;
+        uint32_t ref = 0u, cnt = 0u;
+        if (node < b.n_leaves - 1u) {   // slot lane % 4 of node lane / 4
+            const float4* p = b.quad + 8 * (size_t)node + 2u * (lane & 2u);
+            const float4 r0 = __ldg(p), r1 = __ldg(p + 1), r2 = __ldg(p + 2), r3 = __ldg(p + 3);
+            const bool hi = (lane & 1u) != 0u;
+            ref = __float_as_uint(hi ? r3.y : r3.x);
+            cnt = __float_as_uint(hi ? r3.w : r3.z);
+            if (bvh_slot_ok(b, ref, cnt)) {
+                const float cx = hi ? r0.y : r0.x, cy = hi ? r0.w : r0.z, cz = hi ? r1.y : r1.x;
+                const float hx = hi ? r1.w : r1.z, hy = hi ? r2.y : r2.x, hz = hi ? r2.w : r2.z;
+                // rounded up past the float error of the sum of squares and the root
+                const float rb = sqrtf(hx * hx + hy * hy + hz * hz) * 1.000001f + 1e-6f;
+                pass = cone_meets(cone, mk3(cx - o.x, cy - o.y, cz - o.z), rb, rb, 0.0f);
+            }
+        }
+        const uint32_t inner = __ballot_sync(kFull, pass && cnt == 0u);
+        uint32_t leaves = __ballot_sync(kFull, pass && cnt != 0u);
+        if (sp + (uint32_t)__popc(inner) > kWalkStack) return kNoTileList;
+        if ((inner >> lane) & 1u) stack[sp + (uint32_t)__popc(inner & below)] = ref;
+        sp += (uint32_t)__popc(inner);
+        __syncwarp();
+        while (leaves) {
+            const int k = __ffs(leaves) - 1;
+            leaves &= leaves - 1u;
+            const int k2 = leaves ? __ffs(leaves) - 1 : k;
+            uint32_t first = __shfl_sync(kFull, ref, k), c = __shfl_sync(kFull, cnt, k);
+            const uint32_t first2 = __shfl_sync(kFull, ref, k2), c2 = __shfl_sync(kFull, cnt, k2);
+            uint32_t q = lane;
+            if (k2 != k && c <= 16u && c2 <= 16u) {   // lanes 16.. take the next cluster
+                leaves &= leaves - 1u;
+                if (lane >= 16u) first = first2, c = c2, q = lane - 16u;
+            }
+            c = min(c, b.n_leaves - first);
+            bool meets = false;
+            if (q < c) {
+                const float4 s = __ldg(&b.leaf_sph[first + q]);
+                meets = cone_meets(cone, mk3(s.x - o.x, s.y - o.y, s.z - o.z), cone_radius(s.w), 0.0f, 0.0f);
+            }
+            const uint32_t bits = __ballot_sync(kFull, meets);
+            if (count + (uint32_t)__popc(bits) > kTileListMax) return kNoTileList;
+            const uint32_t at = count + (uint32_t)__popc(bits & below);
+            if (FILL && meets && at < cap) out[at] = first + q;
+            count += (uint32_t)__popc(bits);
+        }
+    }
+    return count;
+}
+
 // Primary nearest hit once per pixel of the wave (shared by its samples).
-// With the brute-force tables a warp's 32 neighbouring primary rays share the
-// camera as apex and a narrow cone of directions, so the warp culls the
-// sphere table against the cone first (nearest_cone).
+// A warp's 32 neighbouring primary rays share the camera as apex and a narrow
+// cone of directions, so the candidates are found once per warp:
+//   the camera's tile mask or candidate list where it has them (a camera that
+//   stayed put) and the warp's pixels are one tile;
+//   else, on the brute-force tables, every sphere's cap (worked out by the
+//   block beforehand, cone_cap) against the warp's cone: 15 instructions
+//   a sphere against 45 when each warp works the caps out itself (k_primary of
+//   1920x1080 pixels with 256 spheres 59 -> 40 us);
+//   else, on the LBVH, a walk of the warp's cone into a list in shared memory.
+//   The rays' own walks pay for the same nodes 32 times over, diverging
+//   (3840x2160 pixels over 65,536 spheres: 16.3 -> 1.25 ms); they remain for
+//   warps without a cone or with more candidates than the list holds.
 // With per-(pixel, light) shadow rays (wave_light_vis) it also clears the
 // pixel's visibility word, stores at the pixel's hit slot the hit point with
 // its sphere and the shadow-ray origin with the pixel, and queues in q[0], as
 // bounce 0's shadow rays, one entry (hit slot, light) per distinct light the
 // pixel's samples pick (q[0] is idle until the second bounce).
+constexpr uint32_t kCapSpheres = kTileMaskMaxSpheres;   // caps a block keeps (24 B each)
+constexpr uint32_t kWalkList = 512;                     // candidates a warp's walk keeps (2 KB)
+
 template <int IS>
 __global__ void __launch_bounds__(kThreads) k_primary(SceneView sc, CameraView cam, WaveState ws, WaveJob job)
 {
-    constexpr bool SMEM = IS == kIsSmem;
-    extern __shared__ float4 s_sph[];
+    extern __shared__ float4 s_dyn[];   // caps, or a candidate list per warp (primary_smem)
     const uint32_t n = job.n_pixels;
     if (blockIdx.x * blockDim.x >= n) return;
     const bool cached = job.prim_cached != 0;   // uniform: only the hit queue is built
-    if (SMEM && !cached) stage_spheres(sc, s_sph);
-    const float4* sph = SMEM ? s_sph : sc.sph;
     const float3 o = mk3(cam.pos[0], cam.pos[1], cam.pos[2]);
+    const bool caps = IS != kIsBvh && !cached && !cam.masks && sc.n_sph <= kCapSpheres;   // uniform
+    float2* cap2 = reinterpret_cast<float2*>(s_dyn + sc.n_sph);
+    if (caps) stage_caps(sc.sph, sc.n_sph, o, s_dyn, cap2);
+    const bool walk = IS == kIsBvh && !cached && !cam.tile_info && sc.bvh.n_leaves > sc.bvh.leaf_size;   // uniform
+    uint32_t* list = reinterpret_cast<uint32_t*>(s_dyn) + (threadIdx.x >> 5) * (kWalkList + kWalkStack);
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t* hits = &ws.counters[2 * ((uint32_t)job.max_bounces + 1u)];
     uint2* prim = job.prim_cache ? job.prim_cache + job.pixel0 : ws.prim;
@@ -161,15 +257,50 @@ __global__ void __launch_bounds__(kThreads) k_primary(SceneView sc, CameraView c
             const uint32_t tile_px = job.pixel0 + warp_j;
             const bool tiled = warp_j < n && (tile_px & 31u) == 0u;
             WarpCone cone;
-            uint2 ti = make_uint2(0u, kNoTileList);
-            if (IS == kIsBvh && cam.tile_info && tiled) ti = __ldg(&cam.tile_info[tile_px >> 5]);
-            if (IS == kIsBvh && ti.y != kNoTileList)
-                id = nearest_listed(sc.bvh, cam.tile_lists + ti.x, ti.y, o, d, me, t);
-            else if (IS != kIsBvh && cam.masks && tiled)
-                id = nearest_masked<SMEM>(sph, cam.masks + (size_t)(tile_px >> 5) * cam.mask_words, cam.mask_words,
-                                          o, d, me, t);
-            else if (IS != kIsBvh && warp_cone(me, d, cone)) id = nearest_cone<SMEM>(sph, sc.n_sph, o, d, me, cone, t);
-            else if (me) id = scene_nearest<IS>(sc, sph, o, d, t);
+            if (IS != kIsBvh && cam.masks && tiled) {
+                id = nearest_masked(sc.sph, cam.masks + (size_t)(tile_px >> 5) * cam.mask_words, cam.mask_words, o, d,
+                                    me, t);
+            } else if (IS != kIsBvh && warp_j < n) {
+                bool first;
+                const uint32_t groups = row_groups(me, p, cam.width, first);
+                for (uint32_t g = 0; g < groups; ++g) {
+                    const bool in = me && first == (g == 0u);
+                    float tg = 0.0f;
+                    int32_t h = -1;
+                    if (!warp_cone(in, d, cone)) {
+                        if (in) h = nearest_brute<false>(sc.sph, sc.n_sph, o, d, tg);
+                    } else if (caps) {
+                        h = nearest_caps(sc.sph, sc.n_sph, s_dyn, cap2, o, d, in, cone, tg);
+                    } else {
+                        h = nearest_cone(sc.sph, sc.n_sph, o, d, in, cone, tg);
+                    }
+                    if (in) id = h, t = tg;
+                }
+            } else if (IS == kIsBvh && warp_j < n) {
+                uint2 ti = make_uint2(0u, kNoTileList);
+                const uint32_t* from = list;
+                if (walk) {
+                    bool first;
+                    const uint32_t groups = row_groups(me, p, cam.width, first);
+                    ti.y = 0u;
+                    for (uint32_t g = 0; g < groups && ti.y != kNoTileList; ++g) {
+                        if (warp_cone(me && first == (g == 0u), d, cone))
+                            ti.y = tile_walk<true>(sc.bvh, cone, o, list + kWalkList, ti.y, list, kWalkList);
+                        else ti.y = kNoTileList;
+                        if (ti.y > kWalkList) ti.y = kNoTileList;
+                    }
+                    __syncwarp();   // the list is written
+                } else if (cam.tile_info && tiled) {
+                    ti = __ldg(&cam.tile_info[tile_px >> 5]);
+                    from = cam.tile_lists + ti.x;
+                }
+                if (ti.y != kNoTileList) {
+                    id = nearest_listed(sc.bvh, from, ti.y, o, d, me, t);
+                    if (walk) __syncwarp();   // read before the next tile's walk writes it
+                } else if (me) {
+                    id = bvh_nearest(sc, o, d, t);
+                }
+            }
             if (me) prim[j] = make_uint2(__float_as_uint(t), (uint32_t)id);
         }
         // pixels whose primary ray hits get first-bounce paths; the others'
@@ -1070,11 +1201,11 @@ __global__ void k_dir_table(CameraView cam, float4* out)
 }
 
 // Tile masks (CameraView::masks): one warp per tile of 32 pixels builds the
-// cone of their primary directions as k_primary does (warp_cone over the same
-// directions, primary_ray) and sets bit i where cone_meets passes sphere i, or
-// every bit when the cone is too wide, which is what k_primary's per-warp
-// loop would test.  A k_primary warp whose pixels are this tile, or part of
-// it, has its directions inside this cone.
+// cones of their primary directions as k_primary does (row_groups, warp_cone
+// over the same directions, primary_ray) and sets bit i where sphere i's cap
+// meets one of them, or every bit when a cone is too wide.  A
+// k_primary warp whose pixels are this tile, or part of it, has its directions
+// inside these cones.
 __global__ void __launch_bounds__(kThreads) k_tile_masks(SceneView sc, CameraView cam, uint32_t* masks)
 {
     const uint64_t px = (uint64_t)cam.width * cam.height;
@@ -1083,97 +1214,31 @@ __global__ void __launch_bounds__(kThreads) k_tile_masks(SceneView sc, CameraVie
     const uint32_t lane = threadIdx.x & 31u;
     const float3 o = mk3(cam.pos[0], cam.pos[1], cam.pos[2]);
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32u);
+    extern __shared__ float4 s_dyn[];   // caps, as k_primary's
+    float2* cap2 = reinterpret_cast<float2*>(s_dyn + sc.n_sph);
+    stage_caps(sc.sph, sc.n_sph, o, s_dyn, cap2);
     for (uint64_t t = (uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u; t < tiles; t += warps) {
         const uint64_t p = 32u * t + lane;
         const bool me = p < px;
         float3 d = o;
         if (me) d = primary_ray(cam, (uint32_t)p);
-        WarpCone cone;
-        const bool ok = warp_cone(me, d, cone);
-        for (uint32_t w = 0; w < words; ++w) {
-            const uint32_t i = 32u * w + lane;
-            bool pass = false;
-            if (i < sc.n_sph) {
-                const float4 s = __ldg(&sc.sph[i]);
-                pass = !ok || cone_meets(cone, mk3(s.x - o.x, s.y - o.y, s.z - o.z), cone_radius(s.w), 0.0f, 0.0f);
+        bool first;
+        const uint32_t groups = row_groups(me, (uint32_t)p, cam.width, first);
+        for (uint32_t g = 0; g < groups; ++g) {
+            WarpCone cone;
+            const bool ok = warp_cone(me && first == (g == 0u), d, cone);
+            for (uint32_t w = 0; w < words; ++w) {
+                const uint32_t i = 32u * w + lane;
+                const bool pass = i < sc.n_sph && (!ok || cap_in_cone(s_dyn[i], cap2[i], cone));
+                const uint32_t bits = __ballot_sync(kFull, pass);
+                if (lane == 0u) masks[t * words + w] = g ? masks[t * words + w] | bits : bits;
             }
-            const uint32_t bits = __ballot_sync(kFull, pass);
-            if (lane == 0u) masks[t * words + w] = bits;
         }
     }
 }
 
-// Candidate spheres of one tile of an LBVH scene: a warp-cooperative walk of
-// the 4-wide nodes (lbvh.cu k_pack_quads) with the tile's cone.  A slot is
-// entered when the cone meets the ball around its box centre through the box
-// corners, that radius also added to the distance in the float-error margin:
-// this ball, inflated by cone_meets, contains the inflated test ball of every
-// sphere inside the box, so a slot holding a sphere that passes the sphere
-// test is entered.  A leaf cluster's spheres get the sphere test the
-// brute-force masks use, one per lane.  All lanes call it and keep the same
-// stack.  Returns the number of candidates (the first cap of them written to
-// out when FILL), or kNoTileList when the walk overflows its stack or step
-// budget or the list would pass kTileListMax.
-template <bool FILL>
-__device__ uint32_t tile_walk(const BvhView& b, const WarpCone& cone, float3 o, uint32_t* out, uint32_t cap)
-{
-    const uint32_t lane = lane_id();
-    uint32_t stack[kBvhStack];
-    int sp = 0;
-    stack[sp++] = b.root;
-    uint32_t count = 0u;
-    uint32_t budget = 2u * b.n_leaves + 8u;
-    while (sp > 0) {
-        if (budget-- == 0u) return kNoTileList;
-        const uint32_t node = stack[--sp];
-        if (node >= b.n_leaves - 1u) continue;
-        bool pass = false;
-        uint32_t ref = 0u, cnt = 0u;
-        if (lane < 4u) {   // lane k tests slot k
-            const float4* p = b.quad + 8 * (size_t)node + 4 * (lane >> 1);
-            const float4 r0 = __ldg(p), r1 = __ldg(p + 1), r2 = __ldg(p + 2), r3 = __ldg(p + 3);
-            const bool hi = (lane & 1u) != 0u;
-            ref = __float_as_uint(hi ? r3.y : r3.x);
-            cnt = __float_as_uint(hi ? r3.w : r3.z);
-            if (bvh_slot_ok(b, ref, cnt)) {
-                const float cx = hi ? r0.y : r0.x, cy = hi ? r0.w : r0.z, cz = hi ? r1.y : r1.x;
-                const float hx = hi ? r1.w : r1.z, hy = hi ? r2.y : r2.x, hz = hi ? r2.w : r2.z;
-                // rounded up past the float error of the sum of squares and the root
-                const float rb = sqrtf(hx * hx + hy * hy + hz * hz) * 1.000001f + 1e-6f;
-                pass = cone_meets(cone, mk3(cx - o.x, cy - o.y, cz - o.z), rb, rb, 0.0f);
-            }
-        }
-        uint32_t inner = __ballot_sync(kFull, pass && cnt == 0u);
-        uint32_t leaves = __ballot_sync(kFull, pass && cnt != 0u);
-        while (inner) {
-            const int k = __ffs(inner) - 1;
-            inner &= inner - 1u;
-            const uint32_t r = __shfl_sync(kFull, ref, k);
-            if (sp >= kBvhStack) return kNoTileList;
-            stack[sp++] = r;
-        }
-        while (leaves) {
-            const int k = __ffs(leaves) - 1;
-            leaves &= leaves - 1u;
-            const uint32_t first = __shfl_sync(kFull, ref, k);
-            const uint32_t c = min(__shfl_sync(kFull, cnt, k), b.n_leaves - first);
-            bool meets = false;
-            if (lane < c) {
-                const float4 sp4 = __ldg(&b.leaf_sph[first + lane]);
-                meets = cone_meets(cone, mk3(sp4.x - o.x, sp4.y - o.y, sp4.z - o.z), cone_radius(sp4.w), 0.0f, 0.0f);
-            }
-            const uint32_t bits = __ballot_sync(kFull, meets);
-            if (count + (uint32_t)__popc(bits) > kTileListMax) return kNoTileList;
-            const uint32_t at = count + (uint32_t)__popc(bits & ((1u << lane) - 1u));
-            if (FILL && meets && at < cap) out[at] = first + lane;
-            count += (uint32_t)__popc(bits);
-        }
-    }
-    return count;
-}
-
-// One warp per tile: the cone of the tile's primary directions (as k_primary
-// and k_tile_masks build it) and its candidate walk.  FILL: only tiles with a
+// One warp per tile: the cones of the tile's primary directions (as k_primary
+// and k_tile_masks build them) and their candidate walks.  FILL: only tiles with a
 // list, written from lists + info[t].x.
 template <bool FILL>
 __global__ void __launch_bounds__(kThreads) k_tile_lists(SceneView sc, CameraView cam, uint2* info, uint32_t* lists)
@@ -1183,6 +1248,7 @@ __global__ void __launch_bounds__(kThreads) k_tile_lists(SceneView sc, CameraVie
     const uint32_t lane = lane_id();
     const float3 o = mk3(cam.pos[0], cam.pos[1], cam.pos[2]);
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32u);
+    __shared__ uint32_t stacks[kThreads / 32][kWalkStack];
     for (uint64_t t = (uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u; t < tiles; t += warps) {
         uint2 ti = make_uint2(0u, 0u);
         if (FILL) {
@@ -1193,31 +1259,41 @@ __global__ void __launch_bounds__(kThreads) k_tile_lists(SceneView sc, CameraVie
         const bool me = p < px;
         float3 d = o;
         if (me) d = primary_ray(cam, (uint32_t)p);
-        WarpCone cone;
-        const bool ok = warp_cone(me, d, cone);
-        if (FILL) {
-            if (ok) tile_walk<true>(sc.bvh, cone, o, lists + ti.x, ti.y);
-        } else {
-            const uint32_t len = ok ? tile_walk<false>(sc.bvh, cone, o, nullptr, 0u) : kNoTileList;
-            if (lane == 0u) info[t] = make_uint2(0u, len);
+        bool first;
+        const uint32_t groups = row_groups(me, (uint32_t)p, cam.width, first);
+        uint32_t len = 0u;
+        for (uint32_t g = 0; g < groups && len != kNoTileList; ++g) {
+            WarpCone cone;
+            if (warp_cone(me && first == (g == 0u), d, cone))
+                len = tile_walk<FILL>(sc.bvh, cone, o, stacks[threadIdx.x / 32u], len, FILL ? lists + ti.x : nullptr,
+                                      ti.y);
+            else len = kNoTileList;
         }
+        if (!FILL && lane == 0u) info[t] = make_uint2(0u, len);
     }
 }
 
-// Offsets of the tile lists: one block, chunks of kThreads tiles in order;
-// tiles past 2^31 - 1 listed entries in all lose their list.
-__global__ void __launch_bounds__(kThreads) k_tile_list_scan(uint2* info, uint64_t tiles, uint32_t* total)
+// Offsets of the tile lists: one block of 1,024 threads, kScanItems tiles a
+// thread and step, in order; tiles past 2^31 - 1 listed entries in all lose
+// their list.  The steps are a serial chain: 259,200 tiles one per thread of
+// 256 were 742 us, this is 233 us.
+constexpr int kScanThreads = 1024;
+constexpr int kScanItems = 8;
+
+__global__ void __launch_bounds__(kScanThreads) k_tile_list_scan(uint2* info, uint64_t tiles, uint32_t* total)
 {
-    __shared__ uint32_t warp_sums[kThreads / 32];
-    __shared__ uint64_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
+    __shared__ uint32_t warp_sums[kScanThreads / 32];
     const uint32_t lane = lane_id(), w = threadIdx.x / 32u;
-    for (uint64_t base = 0; base < tiles; base += kThreads) {
-        const uint64_t i = base + threadIdx.x;
-        uint2 ti = i < tiles ? info[i] : make_uint2(0u, 0u);
-        const uint32_t v = ti.y == kNoTileList ? 0u : ti.y;
-        uint32_t x = v;
+    uint64_t carry = 0;   // the same on every thread
+    for (uint64_t base = 0; base < tiles; base += (uint64_t)kScanThreads * kScanItems) {
+        const uint64_t i0 = base + (uint64_t)threadIdx.x * kScanItems;
+        uint32_t len[kScanItems], sum = 0u;   // at most kScanItems * kTileListMax
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            len[k] = i0 + k < tiles ? info[i0 + k].y : 0u;
+            sum += len[k] == kNoTileList ? 0u : len[k];
+        }
+        uint32_t x = sum;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
             const uint32_t y = __shfl_up_sync(kFull, x, off);
@@ -1225,17 +1301,23 @@ __global__ void __launch_bounds__(kThreads) k_tile_list_scan(uint2* info, uint64
         }
         if (lane == 31u) warp_sums[w] = x;
         __syncthreads();
-        uint64_t pre = carry;
-        for (uint32_t k = 0; k < w; ++k) pre += warp_sums[k];
-        const uint64_t at = pre + x - v;
-        if (i < tiles) {
-            if (at + v > 0x7fffffffull) ti.y = kNoTileList;
-            ti.x = ti.y == kNoTileList ? 0u : (uint32_t)at;
-            info[i] = ti;
+        uint32_t pre = 0u, all = 0u;
+        for (uint32_t k = 0; k < kScanThreads / 32; ++k) {
+            const uint32_t v = warp_sums[k];
+            pre += k < w ? v : 0u;
+            all += v;
         }
-        __syncthreads();
-        if (threadIdx.x == kThreads - 1) carry = pre + x;
-        __syncthreads();
+        uint64_t at = carry + pre + x - sum;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            if (i0 + k >= tiles) break;
+            uint32_t v = len[k] == kNoTileList ? 0u : len[k];
+            const bool none = len[k] == kNoTileList || at + v > 0x7fffffffull;
+            info[i0 + k] = make_uint2(none ? 0u : (uint32_t)at, none ? kNoTileList : v);
+            at += v;
+        }
+        carry += all;
+        __syncthreads();   // warp_sums is read before the next step writes it
     }
     if (threadIdx.x == 0) *total = (uint32_t)(carry < 0x7fffffffull ? carry : 0x7fffffffull);
 }
@@ -1277,14 +1359,22 @@ void with_mode(int mode, F&& f)
     else f(std::integral_constant<int, kIsGlobal>{});
 }
 
+// k_primary's dynamic shared memory: the caps of a brute-force table, or a
+// candidate list and a walk's stack per warp; none when the camera has its
+// masks or lists.
+size_t primary_smem(int mode, uint32_t n_sph, int threads, bool lists)
+{
+    if (mode == kIsBvh) return lists ? 0 : (size_t)(threads / 32) * (kWalkList + kWalkStack) * sizeof(uint32_t);
+    return !lists && n_sph <= kCapSpheres ? n_sph * (sizeof(float4) + sizeof(float2)) : 0;
+}
+
 template <int IS>
-cudaError_t occupancy(int threads, size_t bytes, int* ext, int* sh, int* pr)
+cudaError_t occupancy(uint32_t n_sph, int threads, size_t bytes, int* ext, int* sh, int* pr)
 {
     if (bytes > 48 * 1024) {
         const int b = (int)bytes;
         const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
         cudaError_t e = cudaFuncSetAttribute(k_bounce<IS>, a, b);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_primary<IS>, a, b);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_shadow<IS, false>, a, b);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_shadow<IS, true>, a, b);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace<IS>, a, b);
@@ -1292,7 +1382,9 @@ cudaError_t occupancy(int threads, size_t bytes, int* ext, int* sh, int* pr)
     }
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ext, k_bounce<IS>, kExtendThreads, bytes);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(sh, k_shadow<IS, false>, threads, bytes);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(pr, k_primary<IS>, threads, bytes);
+    constexpr int PIS = IS == kIsBvh ? kIsBvh : kIsGlobal;
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(pr, k_primary<PIS>, threads, primary_smem(IS, n_sph, threads, false));
     return e;
 }
 
@@ -1307,7 +1399,7 @@ cudaError_t plan_launch(const SceneView& sc, int device, int threads, LaunchShap
     const int mode = isect_mode(sc);
     const size_t bytes = mode == kIsSmem ? smem_table_bytes(sc.n_sph) : 0;
     int ext = 0, sh = 0, pr = 0;
-    with_mode(mode, [&](auto m) { e = occupancy<decltype(m)::value>(threads, bytes, &ext, &sh, &pr); });
+    with_mode(mode, [&](auto m) { e = occupancy<decltype(m)::value>(sc.n_sph, threads, bytes, &ext, &sh, &pr); });
     if (e != cudaSuccess) return e;
     out->threads = threads;
     out->blocks_extend = sms * (ext > 0 ? ext : 1);
@@ -1350,7 +1442,9 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
             constexpr int IS = decltype(m)::value;
             const int gp = grid_for(job.n_pixels, shape.threads, shape.blocks_primary);
             begin(kFamExtend);
-            k_primary<IS><<<gp, shape.threads, sm, stream>>>(sc, cam, ws, job);
+            k_primary<IS == kIsBvh ? kIsBvh : kIsGlobal>
+                <<<gp, shape.threads, primary_smem(shape.mode, sc.n_sph, shape.threads, cam.masks || cam.tile_info), stream>>>(
+                    sc, cam, ws, job);
             end(kFamExtend);
             ++nl;
             if (vis) {   // bounce 0's shadow rays, one per (pixel, light), before the shading
@@ -1442,7 +1536,8 @@ cudaError_t enqueue_tile_masks(const SceneView& sc, const CameraView& cam, uint3
     const uint64_t px = (uint64_t)cam.width * cam.height;
     if (px == 0 || sc.n_sph == 0 || sc.n_sph > kTileMaskMaxSpheres) return cudaErrorInvalidValue;
     const uint64_t tiles = (px + 31u) / 32u;
-    k_tile_masks<<<grid_for(tiles * 32u, kThreads, 4096), kThreads, 0, stream>>>(sc, cam, masks);
+    k_tile_masks<<<grid_for(tiles * 32u, kThreads, 1024), kThreads, primary_smem(kIsGlobal, sc.n_sph, kThreads, false),
+                   stream>>>(sc, cam, masks);
     return cudaGetLastError();
 }
 
@@ -1453,7 +1548,7 @@ cudaError_t enqueue_tile_list_counts(const SceneView& sc, const CameraView& cam,
     if (px == 0 || !sc.use_bvh || sc.bvh.n_leaves < 2) return cudaErrorInvalidValue;
     const uint64_t tiles = (px + 31u) / 32u;
     k_tile_lists<false><<<grid_for(tiles * 32u, kThreads, 4096), kThreads, 0, stream>>>(sc, cam, info, nullptr);
-    k_tile_list_scan<<<1, kThreads, 0, stream>>>(info, tiles, total);
+    k_tile_list_scan<<<1, kScanThreads, 0, stream>>>(info, tiles, total);
     return cudaGetLastError();
 }
 
