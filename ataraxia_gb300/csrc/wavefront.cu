@@ -14,8 +14,8 @@
 //   shadow rays are tested right after the shading and a continuation ray is
 //   traced where it is made, so only rays that hit are queued:
 //   k_shade          bounce 1: shades its queue of hits on full warps.
-//   k_paths          bounces >= 2 in one persistent launch: each block
-//                    carries a pool of paths to the end.
+//   k_paths          bounces >= 2 in one persistent launch: each lane
+//                    carries a path to its end, then takes the next.
 //   k_shadow         any-hit over a shadow queue: the first bounce's (pixel,
 //                    light) rays, and per-sample shadow rays of LBVH scenes.
 //   k_accumulate     adds the wave's per-sample colours to the float4
@@ -714,93 +714,72 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
 }
 
 // The sparse late bounces (b >= b0) of scenes with a light buffer in one
-// persistent launch: a block keeps a pool of paths (path id and bounce) whose
-// next ray hits, in shared memory, refilled with chunks of bounce b0's queue
-// (one atomic claim per chunk), and carries each path through all its
-// remaining bounces: a round shades up to a block of pool paths on full
-// warps, traces their continuations and puts those that hit back into the
-// pool.  Late bounces hold few rays, so separate launches would be mostly
-// launch latency and tails.  A path's bounces run in order in one block, so
-// its colour sums are in the reference's order.
+// persistent launch: a lane carries a path of bounce b0's queue, whose next ray
+// hits, through all its remaining bounces in registers, and takes the next one
+// of its warp's share when it ends, so warps stay full while the queue lasts.
+// Late bounces hold few rays: as launches of their own they would be mostly
+// launch latency and tails, and what is left is a chain of bounces, each a few
+// dependent loads.  A block-wide pool of paths refilled between barriers took
+// 37 us for a lane of the medium scene (8.3 M paths), this 31.  A path's bounces
+// run in order in one thread, so its colour sums are in the reference's order.
 template <int IS>
 __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
     k_paths(SceneView sc, WaveState ws, WaveJob job, int b0)
 {
-    constexpr bool SMEM = IS == kIsSmem;
-    constexpr uint32_t kPool = 2u * kExtendThreads;
-    extern __shared__ float4 s_sph[];
-    __shared__ uint32_t p_pid[kPool];
-    __shared__ uint16_t p_bounce[kPool];   // bounces are at most 4096
-    __shared__ uint32_t p_n, chunk;
-    __shared__ bool dry;                      // bounce b0's queue is used up
-    const uint32_t n0 = ws.counters[2 * b0];  // bounce b0's queue
-    if (n0 == 0u) return;
-    if (SMEM) stage_spheres(sc, s_sph);   // ends with a barrier
-    const float4* sph = SMEM ? s_sph : sc.sph;
+    const uint32_t n0 = ws.counters[2 * b0];   // bounce b0's queue
+    const uint32_t lane = lane_id();
+    // the warp's share: chunks of 32 entries, one in every grid's worth of warps
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    uint32_t chunk = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u, used = 0u;   // warp-uniform
+    if (chunk * 32u >= n0) return;
     const uint32_t* q0 = (b0 & 1) ? ws.q[1] : ws.q[0];
-    uint32_t* claim = &ws.counters[2 * ((uint32_t)job.max_bounces + 1u) + 2u];
     uint32_t rays = 0u, traced = 0u;   // this thread's continuation rays, shadow rays
-    if (threadIdx.x == 0) {
-        p_n = 0u;
-        dry = false;
-    }
-    __syncthreads();
+    bool live = false;
+    uint32_t pid = 0u, b = 0u, seed = 0u;
+    float3 o = mk3(0.f, 0.f, 0.f), d = o, thr = o;
+    int32_t hit = -1;
+    float tmin = 0.0f;
 
-    for (;;) {   // ends: every round takes paths off the pool, which only the queue refills
-        if (!dry && p_n < blockDim.x) {   // block-uniform: refill from bounce b0's queue
-            if (threadIdx.x == 0) {
-                chunk = atomicAdd(claim, blockDim.x);
-                dry = chunk >= n0;
+    for (;;) {   // ends: every round takes each live path a bounce further or off
+        uint32_t idle = __ballot_sync(kFull, !live);
+        while (idle && chunk * 32u < n0) {   // lanes without a path take the next of the share
+            const uint32_t have = min(32u, n0 - chunk * 32u) - used;
+            const uint32_t rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (!live && rank < have) {
+                pid = q0[chunk * 32u + used + rank];
+                const float4 ro = ws.ray_o[pid];
+                const float4 rd = ws.ray_d[pid];
+                const float4 tt = ws.thr[pid];
+                o = mk3(ro.x, ro.y, ro.z);
+                seed = __float_as_uint(ro.w);
+                d = mk3(rd.x, rd.y, rd.z);
+                tmin = rd.w;
+                thr = mk3(tt.x, tt.y, tt.z);
+                hit = (int32_t)__float_as_uint(tt.w);
+                b = (uint32_t)b0;
+                live = true;
             }
-            __syncthreads();
-            const uint32_t c0 = chunk;
-            if (c0 < n0) {
-                const uint32_t take = min(blockDim.x, n0 - c0), at = p_n;
-                if (threadIdx.x < take) {
-                    p_pid[at + threadIdx.x] = q0[c0 + threadIdx.x];
-                    p_bounce[at + threadIdx.x] = (uint16_t)b0;
-                }
-                __syncthreads();
-                if (threadIdx.x == 0) p_n = at + take;
+            const uint32_t took = min((uint32_t)__popc(idle), have);
+            used += took;
+            if (used == min(32u, n0 - chunk * 32u)) {
+                chunk += warps;
+                used = 0u;
             }
-            __syncthreads();
+            idle = __ballot_sync(kFull, !live);
         }
-        const uint32_t np = p_n;
-        if (np == 0u) break;
-
-        // shade up to a block of pool paths (from the top of the pool)
-        const uint32_t take = min(np, blockDim.x);
-        uint32_t pid = 0u, b = 0u;
-        if (threadIdx.x < take) {
-            pid = p_pid[np - 1u - threadIdx.x];
-            b = p_bounce[np - 1u - threadIdx.x];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) p_n = np - take;
-        __syncthreads();
-
-        Shaded r{};
-        uint32_t seed = 0u, own = ~0u;
-        float3 o = mk3(0.f, 0.f, 0.f), d = o, thr = o;
-        int32_t nhit = -1;
-        float nt = 0.0f;
-        if (threadIdx.x < take) {
-            const float4 ro = ws.ray_o[pid];
-            const float4 rd = ws.ray_d[pid];
-            const float4 tt = ws.thr[pid];
-            o = mk3(ro.x, ro.y, ro.z);
-            seed = __float_as_uint(ro.w) + b;
-            d = mk3(rd.x, rd.y, rd.z);
-            thr = mk3(tt.x, tt.y, tt.z);
+        if (idle == kFull) break;
+        if (live) {
+            Shaded r{};
+            uint32_t own = ~0u;
+            seed += b;
             const bool last = (int)b + 1 >= job.max_bounces;
-            shade_hit<SMEM, true>(sc, sph, ws, pid, (int32_t)__float_as_uint(tt.w), rd.w, o, d, thr, own, seed, last,
-                                  false, 0u, r);
+            shade_hit<false, true>(sc, sc.sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, false, 0u, r);
             traced += r.traced_sh ? 1u : 0u;
             bool sky = false;
             if (r.push_next) {
                 ++rays;
-                nhit = scene_nearest_from<IS>(sc, sph, own, o, d, nt);
-                r.push_next = nhit >= 0;
+                hit = scene_nearest_from<IS>(sc, sc.sph, own, o, d, tmin);
+                r.push_next = hit >= 0;
                 sky = !r.push_next && job.sky;
             }
             if (r.touch || r.lit || sky) {
@@ -809,18 +788,9 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
                 if (sky) c = sky_term(c, thr);
                 ws.col[pid] = make_float4(c.x, c.y, c.z, c0.w);
             }
-            if (r.push_next) {
-                ws.ray_o[pid] = make_float4(o.x, o.y, o.z, __uint_as_float(seed));
-                ws.ray_d[pid] = make_float4(d.x, d.y, d.z, nt);
-                ws.thr[pid] = make_float4(thr.x, thr.y, thr.z, __uint_as_float((uint32_t)nhit));
-            }
+            live = r.push_next;
+            ++b;
         }
-        const uint32_t k = warp_push(&p_n, r.push_next);
-        if (r.push_next) {
-            p_pid[k] = pid;
-            p_bounce[k] = (uint16_t)(b + 1u);
-        }
-        __syncthreads();
     }
     // statistics: every continuation ray traced here, shadow rays into bounce
     // b0's slot (only sums over bounces are read)

@@ -200,7 +200,7 @@ constexpr uint64_t kWaveBytesPerPath = 7 * 16 + 4 * 4 + 8;
 constexpr uint64_t kWaveArrays = 12;
 
 // Counter slots after the per-bounce pairs: [2*(max_bounces+1)] = hit pixels
-// (the next one is unused), [2*(max_bounces+1)+2] = rays of k_paths' starting queue claimed so far,
+// (the next two are unused),
 // [2*(max_bounces+1)+3] = extension rays traced that no queue counts (with a
 // light buffer a ray is traced where it is made and only hits are queued:
 // the misses, and every ray k_paths traces).
