@@ -20,7 +20,7 @@ constexpr uint32_t kDefaultBvhThreshold = 1025;  // LBVH above the direction buf
 double pass_cost(const SceneView& sc, uint64_t paths, int32_t bounces)
 {
     const double b = std::max(0, bounces);
-    const double per_ray = sc.use_bvh ? 100.0 * std::log2((double)sc.n_sph + 2.0) : (double)sc.n_sph + 8.0;
+    const double per_ray = sc.use_bvh && sc.db.n == 0 ? 100.0 * std::log2((double)sc.n_sph + 2.0) : (double)sc.n_sph + 8.0;
     return (double)paths * (1.0 + 0.5 * b) * per_ray + 2.0e7 * (b + 3.0);
 }
 }  // namespace
@@ -249,6 +249,12 @@ atx_status Batch::autotune(uint32_t passes, atx_batch_tuning* chosen)
     for (auto& p : slots_)
         if (p && p->frame != 1) return fail(ATX_ERR_INVALID_ARG, "batch_autotune: scenes must be at frame 1");
     if (!passes) passes = 2;
+    // the trials are passes over the same scenes: lists they would get on the way come first
+    for (auto& p : slots_)
+        if (p && lists_ && p->scene.lists_due(2ull * kDbMaxBvhSpheres * kDbMaxBvhSpheres)) {
+            p->scene.build_lists(&budget_, up_stream_);
+            ATX_CUDA(cudaEventRecord(uploaded_, up_stream_));
+        }
     // lanes x path state per lane (Mi paths); at 136 B per path the largest is ~37 GB
     const uint32_t cand[][2] = {{2, 64}, {4, 32}, {4, 16}, {8, 16}, {8, 32}, {16, 8}, {16, 16}};
     double best = 1e300;
@@ -356,6 +362,10 @@ atx_status Batch::run(cudaEvent_t done)
         const uint64_t px = (uint64_t)s->w * s->h;
         const uint64_t p = px * s->spp_next;
         paths += p;
+        if (lists_ && s->settings.max_bounces > 0 && s->scene.lists_due(p)) {
+            s->scene.build_lists(&budget_, up_stream_);
+            ATX_CUDA(cudaEventRecord(uploaded_, up_stream_));
+        }
         const uint64_t want = (p + tuning_.lane_wave_paths - 1) / tuning_.lane_wave_paths;
         const uint32_t n = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({want, max_lanes, px}));
         const double c = pass_cost(s->scene.view, p, s->settings.max_bounces) / n;

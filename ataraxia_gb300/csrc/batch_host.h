@@ -64,6 +64,10 @@ public:
     // added from now on (0: default_cell_res by sphere count; the server's
     // per-job scenes use kCellResJobs, which are cheaper to build).
     void set_cell_res(uint32_t res) { cell_res_ = res; }
+    // Whether LBVH scenes get light and direction buffers once they have been
+    // rendered enough (SceneStore::lists_due).  The server's jobs do not: their
+    // device bytes are fixed when they are admitted.
+    void set_lists(bool on) { lists_ = on; }
 
 private:
     struct Slot {
@@ -94,6 +98,7 @@ private:
 
     atx_config cfg_;
     uint32_t cell_res_ = 0;
+    bool lists_ = true;
     Budget budget_;      // resident scenes
     Budget scratch_;     // lanes' path state
     cudaStream_t stream_ = nullptr;      // passes, read-backs, frees

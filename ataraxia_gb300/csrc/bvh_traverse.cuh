@@ -183,9 +183,8 @@ __device__ __forceinline__ void bvh_order(float& ta, uint32_t& ra, uint32_t& ca,
 // 31 4-wide levels: 94 entries.
 constexpr int kBvhStack = 96;
 
-__device__ __forceinline__ int32_t bvh_nearest(const SceneView& sc, float3 o, float3 d, float& tmin)
+__device__ __forceinline__ int32_t bvh_nearest(const BvhView& b, float3 o, float3 d, float& tmin)
 {
-    const BvhView& b = sc.bvh;
     const float a = dot3(d, d);
     // tm must start finite: culled slots carry the key +inf, and the leaf loop
     // below ends at the first key beyond tm, so +inf here would run the leaf
@@ -280,9 +279,8 @@ __device__ __forceinline__ int32_t nearest_listed(const BvhView& b, const uint32
     return best;
 }
 
-__device__ __forceinline__ bool bvh_occluded(const SceneView& sc, float3 o, float3 d, float dist2)
+__device__ __forceinline__ bool bvh_occluded(const BvhView& b, float3 o, float3 d, float dist2)
 {
-    const BvhView& b = sc.bvh;
     const float a = dot3(d, d);
     if (b.n_leaves < 2 || b.n_leaves <= b.leaf_size) return leaf_occluded(b, 0u, min(b.n_leaves, 32u), o, d, a, dist2);
     const float3 inv_d = safe_inv(d);
@@ -322,6 +320,18 @@ __device__ __forceinline__ bool bvh_occluded(const SceneView& sc, float3 o, floa
         }
     }
     return false;
+}
+
+// The walks out of line, for kernels that take them rarely (a cell list that
+// overflowed).
+__device__ __noinline__ int32_t bvh_nearest_call(BvhView b, float3 o, float3 d, float* tmin)
+{
+    return bvh_nearest(b, o, d, *tmin);
+}
+
+__device__ __noinline__ bool bvh_occluded_call(BvhView b, float3 o, float3 d, float dist2)
+{
+    return bvh_occluded(b, o, d, dist2);
 }
 
 }  // namespace atx

@@ -215,6 +215,18 @@ __device__ Cap make_cap(float3 o, float reach, float e1, float e2, float4 s, flo
     return c;
 }
 
+__device__ __forceinline__ Cap shfl_cap(const Cap& c, int from)
+{
+    Cap x;
+    x.v.x = __shfl_sync(0xffffffffu, c.v.x, from);
+    x.v.y = __shfl_sync(0xffffffffu, c.v.y, from);
+    x.v.z = __shfl_sync(0xffffffffu, c.v.z, from);
+    x.dist = __shfl_sync(0xffffffffu, c.dist, from);
+    x.sb = __shfl_sync(0xffffffffu, c.sb, from);
+    x.cb = __shfl_sync(0xffffffffu, c.cb, from);
+    return x;
+}
+
 // Whether a cap meets the cone (axis, half-angle with cosine ch and sine sh):
 // cos(angle between the axes) >= cos(half-angle + beta), with a 2e-5 slack.
 __device__ __forceinline__ bool cap_meets(float3 axis, float ch, float sh, const Cap& c)
@@ -222,7 +234,7 @@ __device__ __forceinline__ bool cap_meets(float3 axis, float ch, float sh, const
     return c.sb < 0.0f || dotf3(axis, c.v) >= c.dist * (ch * c.cb - sh * c.sb - 2e-5f);
 }
 
-constexpr uint32_t kFaceCap = 1024;   // caps a block keeps in shared memory (26 B each)
+constexpr uint32_t kFaceCap = 2048;   // caps a block keeps in shared memory (26 B each)
 
 // The cell lists of both buffers: one block of 256 threads per (apex, cube
 // face, share of the face's tiles), the apexes the n_db spheres, then the
@@ -240,16 +252,18 @@ constexpr uint32_t kFaceCap = 1024;   // caps a block keeps in shared memory (26
 // of the face (with its square roots and division) took 680 us for 256 spheres
 // and 8 lights at 32 cells along an edge (1.6 M cells), this takes 47 us; 1,000
 // spheres and 12 lights 5,430 -> 317 us.  Bound by issue; the sectors written
-// are 50 MB for 256 spheres (8 us).
+// are 50 MB for 256 spheres (8 us).  LINE: 16-bit words per cell line.
 // More spheres than kFaceCap on a face: the tiles test all n (worked out on
 // the fly).
+template <uint32_t LINE>
 __global__ void __launch_bounds__(256) k_cells_build(const float4* __restrict__ sph, const float* __restrict__ rad,
                                                      uint32_t n, uint32_t n_db, const float* __restrict__ reach,
                                                      uint16_t* db_line, const DevLight* __restrict__ lights,
                                                      const float* __restrict__ dcap, uint16_t* lb_line, uint32_t res,
                                                      uint32_t face_cap, Cones cones)
 {
-    constexpr uint32_t kRow = kLbLine / 2u + 1u;   // 32-bit words per staged line (odd: no bank conflicts)
+    constexpr uint32_t kRow = LINE / 2u + 1u;      // 32-bit words per staged line (odd: no bank conflicts)
+    constexpr uint32_t kMax = LINE - 1u;           // spheres a line holds
     extern __shared__ float4 s_dyn[];              // face_cap x (v, dist), then (sb, cb), then the indices
     float4* f_v = s_dyn;
     float2* f_sc = reinterpret_cast<float2*>(f_v + face_cap);
@@ -266,13 +280,13 @@ __global__ void __launch_bounds__(256) k_cells_build(const float4* __restrict__ 
         o = make_float3(s.x, s.y, s.z);
         rho = reach[apex];
         e1 = 0.0f, e2 = rho;
-        line = db_line + (size_t)apex * cells_for(res) * kLbLine;
+        line = db_line + (size_t)apex * cells_for(res) * LINE;
     } else {
         const uint32_t l = apex - n_db;
         o = make_float3(lights[l].pos[0], lights[l].pos[1], lights[l].pos[2]);
         rho = dcap[l];
         e1 = 2e-4f, e2 = (float)kK * rho;
-        line = lb_line + (size_t)l * cells_for(res) * kLbLine;
+        line = lb_line + (size_t)l * cells_for(res) * LINE;
     }
 
     // the face's spheres, by an ordered compaction over the block
@@ -339,31 +353,27 @@ __global__ void __launch_bounds__(256) k_cells_build(const float4* __restrict__ 
             while (mask) {   // index order
                 const int k = __ffs(mask) - 1;
                 mask &= mask - 1u;
-                Cap x;
-                x.v.x = __shfl_sync(0xffffffffu, c.v.x, k);
-                x.v.y = __shfl_sync(0xffffffffu, c.v.y, k);
-                x.v.z = __shfl_sync(0xffffffffu, c.v.z, k);
-                x.dist = __shfl_sync(0xffffffffu, c.dist, k);
-                x.sb = __shfl_sync(0xffffffffu, c.sb, k);
-                x.cb = __shfl_sync(0xffffffffu, c.cb, k);
+                const Cap x = shfl_cap(c, k);
                 const uint32_t xi = __shfl_sync(0xffffffffu, id, k);
                 if (cap_meets(ctr, cc.w, sh, x)) {
-                    if (cnt < kLbMaxList) mine[1u + cnt] = (uint16_t)xi;
+                    if (cnt < kMax) mine[1u + cnt] = (uint16_t)xi;
                     ++cnt;
                 }
             }
         }
-        mine[0] = (uint16_t)(cnt > kLbMaxList ? kLbAll : cnt);
-        const bool longer = __any_sync(0xffffffffu, me && cnt > 15u && cnt <= kLbMaxList);
+        mine[0] = (uint16_t)(cnt > kMax ? kLbAll : cnt);
+        const uint32_t listed = me && cnt <= kMax ? cnt : 0u;
+        uint32_t sectors = 1u;   // of 16 words, that the tile's longest list needs
+        while (sectors < LINE / 16u && __any_sync(0xffffffffu, listed >= sectors * 16u)) ++sectors;
         __syncwarp();
-        // eight lanes write a cell's first 32 bytes (15 spheres), and the other
-        // 32 when a list of the tile needs them
-        for (uint32_t half = 0; half < (longer ? 2u : 1u); ++half)
+        // eight lanes write 32 bytes of a cell: the count and 15 spheres, then 16
+        // more where a list of the tile needs them
+        for (uint32_t part = 0; part < sectors; ++part)
             for (uint32_t c0 = 0; c0 < 32u; c0 += 4u) {
-                const uint32_t c = c0 + lane / 8u, w = half * 8u + lane % 8u;
+                const uint32_t c = c0 + lane / 8u, w = part * 8u + lane % 8u;
                 const uint32_t i = i0 + c / kTileJ, j = j0 + c % kTileJ;
                 if (i < res && j < res)
-                    reinterpret_cast<uint32_t*>(line + (size_t)((f * res + i) * res + j) * kLbLine)[w] =
+                    reinterpret_cast<uint32_t*>(line + (size_t)((f * res + i) * res + j) * LINE)[w] =
                         stage[warp][c * kRow + w];
             }
         __syncwarp();
@@ -372,28 +382,30 @@ __global__ void __launch_bounds__(256) k_cells_build(const float4* __restrict__ 
 
 }  // namespace
 
-uint64_t lb_bytes(uint32_t nl, uint32_t res)
+uint64_t lb_bytes(uint32_t nl, uint32_t res, uint32_t line_words)
 {
     const uint64_t cells = (uint64_t)nl * cells_for(res);
-    return up(cells * kLbLine * sizeof(uint16_t)) + up(nl * sizeof(float)) + cone_bytes(res) + 256;
+    return up(cells * line_words * sizeof(uint16_t)) + up(nl * sizeof(float)) + cone_bytes(res) + 256;
 }
 
-uint64_t db_bytes(uint32_t n, uint32_t res)
+uint64_t db_bytes(uint32_t n, uint32_t res, uint32_t line_words)
 {
     const uint64_t cells = (uint64_t)n * cells_for(res);
-    return up(cells * kLbLine * sizeof(uint16_t)) + up(n * sizeof(float)) + cone_bytes(res) + 256;
+    return up(cells * line_words * sizeof(uint16_t)) + up(n * sizeof(float)) + cone_bytes(res) + 256;
 }
 
 cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, const DevLight* lights, uint32_t nl,
-                        uint32_t res, void* lbuf, uint64_t lbytes, LightBufferView* lv, void* dbuf, uint64_t dbytes,
-                        DirBufferView* dv, cudaStream_t stream)
+                        uint32_t res, uint32_t line_words, void* lbuf, uint64_t lbytes, LightBufferView* lv,
+                        void* dbuf, uint64_t dbytes, DirBufferView* dv, cudaStream_t stream)
 {
     const bool lb = lbuf != nullptr, db = dbuf != nullptr;
     if (!lb && !db) return cudaSuccess;
-    if (n == 0 || n > kLbMaxSpheres || res < kCellResMin || res > kCellResMax) return cudaErrorInvalidValue;
-    if (lb && (nl == 0 || nl > kLbMaxLights || lbytes < lb_bytes(nl, res))) return cudaErrorInvalidValue;
-    if (db && (n > kDbMaxSpheres || dbytes < db_bytes(n, res))) return cudaErrorInvalidValue;
-    const uint64_t row = (uint64_t)cells_for(res) * kLbLine * sizeof(uint16_t);
+    if (n == 0 || n > kLbMaxSpheres || res < kCellResMin || res > kBvhLightRes ||
+        (line_words != kLbLine && line_words != kBvhLine))
+        return cudaErrorInvalidValue;
+    if (lb && (nl == 0 || nl > kLbMaxLights || lbytes < lb_bytes(nl, res, line_words))) return cudaErrorInvalidValue;
+    if (db && (n > kDbMaxBvhSpheres || dbytes < db_bytes(n, res, line_words))) return cudaErrorInvalidValue;
+    const uint64_t row = (uint64_t)cells_for(res) * line_words * sizeof(uint16_t);
     uint16_t* lline = static_cast<uint16_t*>(lbuf);
     uint16_t* dline = static_cast<uint16_t*>(dbuf);
     float *dcap = nullptr, *reach = nullptr;
@@ -418,8 +430,10 @@ cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, cons
     const uint32_t blocks = (apex_d + apex_l) * 6u, shares = (tiles_for(res) + 7u) / 8u;
     const uint32_t want = (600u + blocks - 1u) / blocks;
     const dim3 grid(blocks, want < shares ? want : shares);
-    k_cells_build<<<grid, 256, smem, stream>>>(sph, radius, n, apex_d, reach, dline, lights, dcap, lline, res, cap,
-                                               cones);
+    const auto build = line_words == kBvhLine ? k_cells_build<kBvhLine> : k_cells_build<kLbLine>;
+    const cudaError_t e = cudaFuncSetAttribute(build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    build<<<grid, 256, smem, stream>>>(sph, radius, n, apex_d, reach, dline, lights, dcap, lline, res, cap, cones);
     if (lb) *lv = LightBufferView{lline, dcap, nl, res};
     if (db) *dv = DirBufferView{dline, reach, n, res};
     return cudaGetLastError();

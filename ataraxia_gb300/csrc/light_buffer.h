@@ -12,19 +12,20 @@
 namespace atx {
 
 // Device bytes cells_build needs for the light buffer of nl lights, and for
-// the direction buffer of n spheres, at res cells along a face's edge.
-uint64_t lb_bytes(uint32_t nl, uint32_t res);
-uint64_t db_bytes(uint32_t n, uint32_t res);
+// the direction buffer of n spheres, at res cells along a face's edge and
+// line_words 16-bit words per cell (kLbLine, or kBvhLine for LBVH scenes).
+uint64_t lb_bytes(uint32_t nl, uint32_t res, uint32_t line_words = kLbLine);
+uint64_t db_bytes(uint32_t n, uint32_t res, uint32_t line_words = kLbLine);
 
 // Builds, on stream, for the n spheres sph (cx, cy, cz, r*r) with radii
-// radius[], at res cells along a face's edge (kCellResMin..kCellResMax):
+// radius[], at res cells along a face's edge (kCellResMin..kBvhLightRes):
 //   the light buffer of the nl lights (1 <= nl <= kLbMaxLights, n <=
-//   kLbMaxSpheres) into lbuf (lb_bytes(nl, res) bytes of device memory; null:
-//   none), *lv its view;
-//   the direction buffer (n <= kDbMaxSpheres) into dbuf (db_bytes(n, res)
-//   bytes; null: none), *dv its view.
+//   kLbMaxSpheres) into lbuf (lb_bytes() of device memory; null: none), *lv
+//   its view;
+//   the direction buffer (n <= kDbMaxBvhSpheres) into dbuf (db_bytes(); null:
+//   none), *dv its view.
 cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, const DevLight* lights, uint32_t nl,
-                        uint32_t res, void* lbuf, uint64_t lbytes, LightBufferView* lv, void* dbuf, uint64_t dbytes,
-                        DirBufferView* dv, cudaStream_t stream);
+                        uint32_t res, uint32_t line_words, void* lbuf, uint64_t lbytes, LightBufferView* lv,
+                        void* dbuf, uint64_t dbytes, DirBufferView* dv, cudaStream_t stream);
 
 }  // namespace atx

@@ -36,6 +36,18 @@ struct SceneStore {
     uint32_t cells() const;
     // Builds the light and direction buffers of the uploaded tables at cell_res.
     atx_status build_cells(Budget* budget, cudaStream_t stream);
+    // Light and direction buffers for an LBVH scene of up to kDbMaxBvhSpheres
+    // spheres, on top of its tree.  Every pair of spheres is looked at, so they
+    // are built only for a scene that goes on being rendered: lists_due counts
+    // the paths about to be traced and says when those so far would have paid
+    // for the build; a scene rendered once, or uploaded for every render, keeps
+    // to the tree.  build_lists leaves the scene on the tree when a budget is
+    // set, which later buffers may need in full, or when the lists would take
+    // more than a quarter of the device's free memory.
+    bool lists_due(uint64_t paths);
+    void build_lists(Budget* budget, cudaStream_t stream);
+    uint64_t paths_seen = 0;    // since the upload, until the lists were tried
+    bool lists_tried = false;
     uint64_t device_bytes() const
     {
         return sph.bytes() + sph_mat.bytes() + sph_rad.bytes() + mat.bytes() + lights.bytes() + bvh.bytes() +

@@ -36,7 +36,11 @@ bool finite3(const float* v) { return std::isfinite(v[0]) && std::isfinite(v[1])
 // and its read-backs; result buffers are page-locked, cached by size.
 class BatchExecutor : public Executor {
 public:
-    explicit BatchExecutor(const atx_config& cfg) : b_(cfg), device_(cfg.device) { b_.set_cell_res(kCellResJobs); }
+    explicit BatchExecutor(const atx_config& cfg) : b_(cfg), device_(cfg.device)
+    {
+        b_.set_cell_res(kCellResJobs);
+        b_.set_lists(false);
+    }
     ~BatchExecutor() override
     {
         if (cudaSetDevice(device_) != cudaSuccess) return;

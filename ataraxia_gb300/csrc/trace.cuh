@@ -438,6 +438,40 @@ __device__ __forceinline__ int32_t nearest_caps(const float4* __restrict__ sph, 
     return best;
 }
 
+template <int IS, bool EXIT = false>
+__device__ __forceinline__ int32_t scene_nearest(const SceneView& sc, const float4* sph, float3 o, float3 d,
+                                                 float& tmin)
+{
+    if (IS == kIsBvh) return bvh_nearest(sc.bvh, o, d, tmin);
+    return nearest_brute<IS == kIsSmem, EXIT>(sph, sc.n_sph, o, d, tmin);
+}
+
+template <int IS, bool EXIT = false>
+__device__ __forceinline__ bool scene_occluded(const SceneView& sc, const float4* sph, float3 o, float3 d,
+                                               float dist2)
+{
+    if (IS == kIsBvh) return bvh_occluded(sc.bvh, o, d, dist2);
+    return occluded_brute<IS == kIsSmem, EXIT>(sph, sc.n_sph, o, d, dist2);
+}
+
+// The same over every sphere, as the way out of a cell list.
+template <int IS>
+__device__ __forceinline__ int32_t all_nearest(const SceneView& sc, const float4* sph, float3 o, float3 d, float& tmin)
+{
+    if (IS != kIsBvh) return scene_nearest<IS>(sc, sph, o, d, tmin);
+    float t;
+    const int32_t id = bvh_nearest_call(sc.bvh, o, d, &t);
+    tmin = t;
+    return id;
+}
+
+template <int IS>
+__device__ __forceinline__ bool all_occluded(const SceneView& sc, const float4* sph, float3 o, float3 d, float dist2)
+{
+    if (IS != kIsBvh) return scene_occluded<IS>(sc, sph, o, d, dist2);
+    return bvh_occluded_call(sc.bvh, o, d, dist2);
+}
+
 // ------------------------------------------------------------ light buffer
 
 // Cell of direction w around a light, as light_buffer.cu lays out the cube:
@@ -489,9 +523,9 @@ __device__ __forceinline__ bool walk_line(const uint16_t* line, uint4 h, uint32_
 
 // Any hit for a shadow ray (o, d, dist2) towards light li: the spheres the
 // light buffer lists for the cell of o seen from the light, or the whole table
-// when that cell overflowed, o lies beyond the buffer's reach or the
-// direction is degenerate.
-template <bool SMEM>
+// (on the LBVH a walk) when that cell overflowed, o lies beyond the buffer's
+// reach or the direction is degenerate.
+template <int IS>
 __device__ __forceinline__ bool occluded_lb(const SceneView& sc, const float4* __restrict__ sph, uint32_t li, float3 o,
                                             float3 d, float dist2)
 {
@@ -499,15 +533,15 @@ __device__ __forceinline__ bool occluded_lb(const SceneView& sc, const float4* _
     const float3 w = mk3(o.x - l0.x, o.y - l0.y, o.z - l0.z);
     const float dc = __ldg(&sc.lb.dcap[li]);
     const int cell = dot3(w, w) <= dc * dc ? lb_cell(w, sc.lb.res) : -1;
-    if (cell < 0) return occluded_brute<SMEM>(sph, sc.n_sph, o, d, dist2);
-    const uint16_t* line = sc.lb.line + ((size_t)li * cells_for(sc.lb.res) + (uint32_t)cell) * kLbLine;
+    if (cell < 0) return all_occluded<IS>(sc, sph, o, d, dist2);
+    const uint16_t* line = sc.lb.line + ((size_t)li * cells_for(sc.lb.res) + (uint32_t)cell) * (IS == kIsBvh ? kBvhLine : kLbLine);
     const uint4 h = __ldg(reinterpret_cast<const uint4*>(line));
     const uint32_t cnt = h.x & 0xffffu;
-    if (cnt == kLbAll) return occluded_brute<SMEM>(sph, sc.n_sph, o, d, dist2);
+    if (cnt == kLbAll) return all_occluded<IS>(sc, sph, o, d, dist2);
     const float a = dot3(d, d);
     return walk_line(line, h, cnt, [&](uint32_t i) {
         float t;
-        return sphere_t(table_sphere<SMEM>(sph, i), o, d, a, t) && t > 0.0f && t * t < dist2;
+        return sphere_t(table_sphere<IS == kIsSmem>(sph, i), o, d, a, t) && t > 0.0f && t * t < dist2;
     });
 }
 
@@ -516,23 +550,23 @@ __device__ __forceinline__ bool occluded_lb(const SceneView& sc, const float4* _
 // the lowest index, as in the brute-force loop), or the whole table when own
 // is not covered (~0u: also when the ray's origin lay beyond own's reach,
 // which the shading that made the ray checks), the cell overflowed or d is
-// degenerate.
-template <bool SMEM>
+// degenerate (on the LBVH a walk then).
+template <int IS>
 __device__ __forceinline__ int32_t nearest_db(const SceneView& sc, const float4* __restrict__ sph, uint32_t own,
                                               float3 o, float3 d, float& tmin)
 {
     const int cell = own < sc.db.n ? lb_cell(d, sc.db.res) : -1;
-    if (cell < 0) return nearest_brute<SMEM>(sph, sc.n_sph, o, d, tmin);
-    const uint16_t* line = sc.db.line + ((size_t)own * cells_for(sc.db.res) + (uint32_t)cell) * kLbLine;
+    if (cell < 0) return all_nearest<IS>(sc, sph, o, d, tmin);
+    const uint16_t* line = sc.db.line + ((size_t)own * cells_for(sc.db.res) + (uint32_t)cell) * (IS == kIsBvh ? kBvhLine : kLbLine);
     const uint4 h = __ldg(reinterpret_cast<const uint4*>(line));
     const uint32_t cnt = h.x & 0xffffu;
-    if (cnt == kLbAll) return nearest_brute<SMEM>(sph, sc.n_sph, o, d, tmin);
+    if (cnt == kLbAll) return all_nearest<IS>(sc, sph, o, d, tmin);
     const float a = dot3(d, d);
     int32_t best = -1;
     float tm = kFltMax;
     walk_line(line, h, cnt, [&](uint32_t i) {
         float t;
-        if (sphere_t(table_sphere<SMEM>(sph, i), o, d, a, t) && t > 0.0f && t < tm) {
+        if (sphere_t(table_sphere<IS == kIsSmem>(sph, i), o, d, a, t) && t > 0.0f && t < tm) {
             tm = t;
             best = (int32_t)i;
         }
@@ -552,29 +586,13 @@ __device__ __forceinline__ bool db_reaches(const SceneView& sc, uint32_t own, fl
     return dot3(e, e) <= reach * reach;
 }
 
-template <int IS, bool EXIT = false>
-__device__ __forceinline__ int32_t scene_nearest(const SceneView& sc, const float4* sph, float3 o, float3 d,
-                                                 float& tmin)
-{
-    if (IS == kIsBvh) return bvh_nearest(sc, o, d, tmin);
-    return nearest_brute<IS == kIsSmem, EXIT>(sph, sc.n_sph, o, d, tmin);
-}
-
 // Nearest hit of a ray leaving sphere own (~0u: from elsewhere).
 template <int IS>
 __device__ __forceinline__ int32_t scene_nearest_from(const SceneView& sc, const float4* sph, uint32_t own, float3 o,
                                                       float3 d, float& tmin)
 {
-    if (IS != kIsBvh && sc.db.n != 0u) return nearest_db<IS == kIsSmem>(sc, sph, own, o, d, tmin);
+    if (sc.db.n != 0u) return nearest_db<IS>(sc, sph, own, o, d, tmin);
     return scene_nearest<IS>(sc, sph, o, d, tmin);
-}
-
-template <int IS, bool EXIT = false>
-__device__ __forceinline__ bool scene_occluded(const SceneView& sc, const float4* sph, float3 o, float3 d,
-                                               float dist2)
-{
-    if (IS == kIsBvh) return bvh_occluded(sc, o, d, dist2);
-    return occluded_brute<IS == kIsSmem, EXIT>(sph, sc.n_sph, o, d, dist2);
 }
 
 }  // namespace atx

@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kThreads) k_primary(SceneView sc, CameraView c
                     id = nearest_listed(sc.bvh, from, ti.y, o, d, me, t);
                     if (walk) __syncwarp();   // read before the next tile's walk writes it
                 } else if (me) {
-                    id = bvh_nearest(sc, o, d, t);
+                    id = bvh_nearest(sc.bvh, o, d, t);
                 }
             }
             if (me) prim[j] = make_uint2(__float_as_uint(t), (uint32_t)id);
@@ -359,12 +359,12 @@ struct Shaded {
 // tested here through the light buffer for INL, else a record for k_shadow),
 // roulette and the next direction, which replace o, d, thr, own and advance
 // seed.
-template <bool SMEM, bool INL>
+template <int IS, bool INL>
 __device__ __forceinline__ void shade_hit(const SceneView& sc, const float4* sph, const WaveState& ws, uint32_t pid,
                                           int32_t hit, float tmin, float3& o, float3& d, float3& thr, uint32_t& own,
                                           uint32_t& seed, bool last, bool vis, uint32_t j, Shaded& r)
 {
-    const float4 s = table_sphere<SMEM>(sph, (uint32_t)hit);
+    const float4 s = table_sphere<IS == kIsSmem>(sph, (uint32_t)hit);
     float3 pos, nrm;
     ray_hit(s, o, d, tmin, pos, nrm);
     const int32_t mi = __ldg(&sc.sph_mat[hit]);
@@ -394,7 +394,7 @@ __device__ __forceinline__ void shade_hit(const SceneView& sc, const float4* sph
             r.lc = c;
         } else if (INL) {   // Renderer.cu:348-352
             const float3 so = add3(pos, muls3(nrm, kOffset));
-            r.lit = sc.n_sph == 0u || !occluded_lb<SMEM>(sc, sph, li, so, L, dist2);
+            r.lit = sc.n_sph == 0u || !occluded_lb<IS>(sc, sph, li, so, L, dist2);
             r.lc = c;
             r.traced_sh = true;
         } else {
@@ -479,7 +479,7 @@ __device__ __forceinline__ void push_hit(const WaveState& ws, uint32_t* qout, ui
 // took 249 us for 1920x1080 on the 256-sphere scene against 59 + 35 us.
 // INL: the scene has a light buffer and shadow rays are tested right after
 // the shading (a lookup and a few spheres) instead of through k_shadow.
-template <bool INL>
+template <int IS, bool INL>
 __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
     k_first(SceneView sc, CameraView cam, WaveState ws, WaveJob job)
 {
@@ -510,12 +510,12 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
             thr = mk3(1.f, 1.f, 1.f);
             seed = p * (job.frame0 + smp);   // bounce 0: seed += 0
             const uint2 pr = prim[j];
-            shade_hit<false, INL>(sc, sc.sph, ws, pid, (int32_t)pr.y, __uint_as_float(pr.x), o, d, thr, own, seed,
+            shade_hit<IS, INL>(sc, sc.sph, ws, pid, (int32_t)pr.y, __uint_as_float(pr.x), o, d, thr, own, seed,
                                   last, vis, j, r);
             float3 c = add3(mk3(0.f, 0.f, 0.f), r.add);
             if (r.lit) c = add3(c, r.lc);   // as k_shadow adds it: after the emission
             if (INL && r.push_next) {
-                nhit = scene_nearest_from<kIsGlobal>(sc, sc.sph, own, o, d, nt);
+                nhit = scene_nearest_from<IS>(sc, sc.sph, own, o, d, nt);
                 r.push_next = nhit >= 0;
                 if (!r.push_next) {
                     ++missed;
@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
             seed = __float_as_uint(ro.w) + (uint32_t)bounce;
             d = mk3(rd.x, rd.y, rd.z);
             thr = mk3(tt.x, tt.y, tt.z);
-            shade_hit<SMEM, false>(sc, sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, false, 0u, r);
+            shade_hit<IS, false>(sc, sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, false, 0u, r);
             if (r.touch || r.lit) {
                 // emission of bounce b, then its light (the order k_shadow adds it in)
                 float4 c = ws.col[pid];
@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
             seed = __float_as_uint(ro.w) + (uint32_t)bounce;
             d = mk3(rd.x, rd.y, rd.z);
             thr = mk3(tt.x, tt.y, tt.z);
-            shade_hit<SMEM, true>(sc, sph, ws, pid, (int32_t)__float_as_uint(tt.w), rd.w, o, d, thr, own, seed, last,
+            shade_hit<IS, true>(sc, sph, ws, pid, (int32_t)__float_as_uint(tt.w), rd.w, o, d, thr, own, seed, last,
                                   false, 0u, r);
             bool sky = false;
             if (r.push_next) {
@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
             uint32_t own = ~0u;
             seed += b;
             const bool last = (int)b + 1 >= job.max_bounces;
-            shade_hit<false, true>(sc, sc.sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, false, 0u, r);
+            shade_hit<IS, true>(sc, sc.sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, false, 0u, r);
             traced += r.traced_sh ? 1u : 0u;
             bool sky = false;
             if (r.push_next) {
@@ -870,7 +870,9 @@ __device__ __forceinline__ void shadow_light(const WaveState& ws, uint32_t idx, 
     ws.col[r.target] = col;
 }
 
-template <int IS, bool VIS>
+// LISTS: an LBVH scene with a light buffer (its walk only for cells that
+// overflowed).
+template <int IS, bool VIS, bool LISTS = false>
 __global__ void __launch_bounds__(kThreads, kShadowBlocksPerSm<IS>) k_shadow(SceneView sc, WaveState ws, int bounce)
 {
     constexpr bool SMEM = IS == kIsSmem;
@@ -886,9 +888,10 @@ __global__ void __launch_bounds__(kThreads, kShadowBlocksPerSm<IS>) k_shadow(Sce
         for (uint32_t idx = first; idx < n; idx += stride) {
             const ShadowRay r = load_shadow<VIS>(sc, ws, idx);
             bool occ;
-            if (IS == kIsBvh) occ = own_occludes(sc, sph, SMEM, r.tag & kShadowSphereMask, r.o, r.d, r.dist2) ||
-                                    scene_occluded<IS>(sc, sph, r.o, r.d, r.dist2);
-            else occ = sc.n_sph != 0u && occluded_lb<SMEM>(sc, sph, r.tag >> 26, r.o, r.d, r.dist2);
+            if (IS == kIsBvh && !LISTS)
+                occ = own_occludes(sc, sph, SMEM, r.tag & kShadowSphereMask, r.o, r.d, r.dist2) ||
+                      scene_occluded<IS>(sc, sph, r.o, r.d, r.dist2);
+            else occ = sc.n_sph != 0u && occluded_lb<IS>(sc, sph, r.tag >> 26, r.o, r.d, r.dist2);
             if (!occ) shadow_light<VIS>(ws, idx, r);
         }
         return;
@@ -1406,8 +1409,7 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
         if (e != cudaSuccess) return e;
         const int g0 = grid_for(paths, kExtendThreads, shape.blocks_extend);
         const bool vis = wave_light_vis(job, sc.n_lights);
-        // a light buffer exists only for the brute-force tables
-        const bool inl = shape.mode != kIsBvh && sc.lb.n_lights != 0u;
+        const bool inl = sc.lb.n_lights != 0u;   // with the LBVH only together with a direction buffer
         with_mode(shape.mode, [&](auto m) {
             constexpr int IS = decltype(m)::value;
             const int gp = grid_for(job.n_pixels, shape.threads, shape.blocks_primary);
@@ -1419,37 +1421,36 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
             ++nl;
             if (vis) {   // bounce 0's shadow rays, one per (pixel, light), before the shading
                 begin(kFamShadow);
-                k_shadow<IS, true><<<shape.blocks_shadow, shape.threads, sm, stream>>>(sc, ws, 0);
+                if constexpr (IS == kIsBvh) {
+                    if (inl) k_shadow<IS, true, true><<<shape.blocks_shadow, shape.threads, 0, stream>>>(sc, ws, 0);
+                    else k_shadow<IS, true><<<shape.blocks_shadow, shape.threads, 0, stream>>>(sc, ws, 0);
+                } else {
+                    k_shadow<IS, true><<<shape.blocks_shadow, shape.threads, sm, stream>>>(sc, ws, 0);
+                }
                 end(kFamShadow);
                 ++nl;
             }
             begin(kFamExtend);
-            if (inl) k_first<true><<<g0, kExtendThreads, 0, stream>>>(sc, cam, ws, job);
-            else k_first<false><<<g0, kExtendThreads, 0, stream>>>(sc, cam, ws, job);
+            constexpr int G = IS == kIsBvh ? kIsBvh : kIsGlobal;   // these read the sphere table through L1
+            if (inl) k_first<G, true><<<g0, kExtendThreads, 0, stream>>>(sc, cam, ws, job);
+            else k_first<kIsGlobal, false><<<g0, kExtendThreads, 0, stream>>>(sc, cam, ws, job);
             end(kFamExtend);
             ++nl;
             for (int b = 0; b < bounces; ++b) {
-                if constexpr (IS != kIsBvh) {
-                    if (inl && b >= kPathsFrom) {   // the late bounces in one persistent launch
-                        // on half the resident blocks: the late bounces are a trickle of
-                        // paths, and the blocks stay resident until their pools drain,
-                        // holding slots the other lanes' kernels could use (+1%)
-                        begin(kFamExtend);
-                        k_paths<kIsGlobal><<<max(1, shape.blocks_extend / 2), kExtendThreads, 0, stream>>>(sc, ws, job,
-                                                                                                           b);
-                        end(kFamExtend);
-                        ++nl;
-                        break;
-                    }
+                if (inl && b >= kPathsFrom) {   // the late bounces in one persistent launch
+                    // on half the resident blocks: the late bounces are a trickle of
+                    // paths, and the blocks stay resident until their pools drain,
+                    // holding slots the other lanes' kernels could use (+1%)
+                    begin(kFamExtend);
+                    k_paths<G><<<max(1, shape.blocks_extend / 2), kExtendThreads, 0, stream>>>(sc, ws, job, b);
+                    end(kFamExtend);
+                    ++nl;
+                    break;
                 }
                 if (b > 0) {
                     begin(kFamExtend);
-                    if constexpr (IS != kIsBvh) {
-                        if (inl) k_shade<kIsGlobal><<<shape.blocks_extend, kExtendThreads, 0, stream>>>(sc, ws, job, b);
-                        else k_bounce<IS><<<shape.blocks_extend, kExtendThreads, sm, stream>>>(sc, ws, job, b);
-                    } else {
-                        k_bounce<IS><<<shape.blocks_extend, kExtendThreads, sm, stream>>>(sc, ws, job, b);
-                    }
+                    if (inl) k_shade<G><<<shape.blocks_extend, kExtendThreads, 0, stream>>>(sc, ws, job, b);
+                    else k_bounce<IS><<<shape.blocks_extend, kExtendThreads, sm, stream>>>(sc, ws, job, b);
                     end(kFamExtend);
                     ++nl;
                 }

@@ -95,6 +95,18 @@ struct LightBufferView {
 // Every extension ray after the first bounce leaves the sphere its path last
 // hit, so its nearest hit tests the spheres of one cell.
 constexpr uint32_t kDbMaxSpheres = 1024;   // 393 KB of cells per sphere at res 32
+// LBVH scenes up to this many spheres get both buffers too, once they have
+// traced enough paths to pay for the build (SceneStore::lists_due), at these
+// resolutions and with lines twice as long (63 spheres).  A lookup and a few
+// spheres replace a walk that runs 5 to 9 of a warp's 32 lanes: 16 samples of
+// 1280x720 pixels over 4,096 spheres 3.28 -> 0.76 ms.  The walk is left for
+// cells whose list overflowed, 0.2% of the extension rays there; with 64-byte
+// lines at 32 cells 1% (1.23 ms), at 16 cells 10%.  Beyond, lists and build
+// grow (442 KB a sphere, every pair looked at) and clusters overflow them.
+constexpr uint32_t kDbMaxBvhSpheres = 4096;
+constexpr uint32_t kBvhDirRes = 24;
+constexpr uint32_t kBvhLightRes = 64;   // a light sees the whole scene behind a cell: finer cells than a sphere's
+constexpr uint32_t kBvhLine = 64;       // 16-bit words per cell
 struct DirBufferView {
     const uint16_t* line;    // [n * cells_for(res) * kLbLine] cell lines, as the light buffer's
     const float* reach;      // [n] the lists hold for ray origins within reach of the sphere's centre
@@ -122,8 +134,8 @@ struct SceneView {
     uint32_t n_lights;
     uint32_t use_bvh;         // 1: traverse bvh instead of the brute-force loop
     BvhView bvh;
-    LightBufferView lb;       // shadow-ray cells of the brute-force tables (lb.n_lights 0: none)
-    DirBufferView db;         // extension-ray cells of the brute-force tables (db.n 0: none)
+    LightBufferView lb;       // shadow-ray cells (lb.n_lights 0: none)
+    DirBufferView db;         // extension-ray cells (db.n 0: none; with the LBVH both or neither)
     uint64_t light_mod;       // fastmod_multiplier(n_lights): x % n_lights by multiplication
 };
 
