@@ -534,7 +534,7 @@ atx_status Renderer::refresh_masks()
     prev_cam_ = camv_;
     prev_cam_valid_ = true;
     if (!same && !still) return ATX_OK;
-    const uint64_t tiles = ((uint64_t)camv_.width * camv_.height + 31u) / 32u;
+    const uint64_t tiles = tile_count(camv_.width, camv_.height);
     if (sc.use_bvh) {
         if (sc.bvh.n_leaves < 2 || sc.bvh.n_leaves <= sc.bvh.leaf_size) return ATX_OK;
         if (!same) {

@@ -210,7 +210,7 @@ __device__ __forceinline__ bool occluded_brute(const float4* __restrict__ sph, u
 // ------------------------------------------------------------- warp cones
 //
 // Rays of one warp that leave one apex in a narrow cone of directions: the
-// primary rays of 32 neighbouring pixels (apex: the camera).  The warp tests every sphere once against the cone of its
+// primary rays of a tile's 32 pixels (apex: the camera).  The warp tests every sphere once against the cone of its
 // active lanes' directions and the lanes run the exact test only on the
 // spheres that pass, in index order; results equal the brute-force loop's.
 //
@@ -252,23 +252,6 @@ __device__ __forceinline__ bool warp_cone(bool me, float3 w, WarpCone& c)
     if (!(c.cos_lo > 0.5f)) return false;
     c.sin_hi = sqrtf(fmaxf(0.0f, 1.0f - c.cos_lo * c.cos_lo)) + 1e-6f;
     return true;
-}
-
-// A warp's 32 consecutive pixels lie in one image row, or at the end of one
-// and the start of the next (and more rows of an image narrower than 32): the
-// lanes of the first row and the others then get a cone each, one after the
-// other.  One cone around both ends of a row is as wide as the image and meets
-// most spheres: with 1279 pixels to a row one warp in 40 tested all of 1,000
-// spheres and its launch waited for it (k_primary with the camera's masks
-// 186 -> 28 us).  Returns how many groups there are and sets first for the
-// lanes of the first.  All 32 lanes call it, lane 0 inside the image; p: the
-// lane's pixel.
-__device__ __forceinline__ uint32_t row_groups(bool me, uint32_t p, uint32_t width, bool& first)
-{
-    const uint32_t row = p / width;
-    const uint32_t row0 = __shfl_sync(0xffffffffu, row, 0);   // by every lane, not behind me
-    first = row == row0;
-    return __any_sync(0xffffffffu, me && !first) ? 2u : 1u;
 }
 
 // Whether a sphere (centre at v from the apex, radius r) may be hit by a ray
@@ -431,6 +414,53 @@ __device__ __forceinline__ int32_t nearest_caps(const float4* __restrict__ sph, 
             if (me && sphere_t(__ldg(&sph[i]), o, d, a, t) && t > 0.0f && t < tm) {
                 tm = t;
                 best = (int32_t)i;
+            }
+        }
+    }
+    tmin = tm;
+    return best;
+}
+
+// Nearest hit among a list of sorted sphere indices of an LBVH scene (a tile's
+// list, or a warp's walk's in shared memory) that holds what every lane's ray
+// can hit.  The warp stages 32 spheres at a time in shared memory (stage, 32
+// float4 of its own, the pair layout of stage_spheres), the brute-force filter
+// marks each lane's candidates and the exact test decides; ties go to the
+// lowest original index, so the list's order does not matter.  Eight
+// instructions a sphere and no branch among them: handing each sphere over by
+// shuffles with the test behind a branch took 27 and a warp's list was a chain
+// of them (287x175 pixels, lists of hundreds in clusters of 7,418 spheres:
+// k_primary 84 -> 42 us).  All 32 lanes call it.
+__device__ __forceinline__ int32_t nearest_listed(const BvhView& b, const uint32_t* list, uint32_t len, float3 o,
+                                                  float3 d, bool me, float4* stage, float& tmin)
+{
+    const float a = dot3(d, d);
+    const uint32_t lane = threadIdx.x & 31u;
+    float* put = reinterpret_cast<float*>(stage + (lane & ~1u)) + (lane & 1u);
+    float tm = kFltMax;
+    int32_t best = -1;
+    for (uint32_t base = 0; base < len; base += 32u) {
+        const uint32_t cnt = min(32u, len - base);
+        const float4 v = __ldg(&b.leaf_sph[list[base + min(lane, cnt - 1u)]]);
+        __syncwarp();   // the chunk before is read
+        put[0] = -v.x;
+        put[2] = -v.y;
+        put[4] = -v.z;
+        put[6] = -v.w;
+        __syncwarp();
+        uint32_t mask = cnt == 32u ? candidate_bits<true, 32>(stage, 0u, o, d, a, 32u)
+                                   : candidate_bits<true, 31, true>(stage, 0u, o, d, a, cnt);
+        if (!me) mask = 0u;
+        while (mask) {
+            const uint32_t k = (uint32_t)__clz(mask);
+            mask &= ~(0x80000000u >> k);
+            float t;
+            if (sphere_t(smem_sphere(stage, k), o, d, a, t) && t > 0.0f) {
+                const int32_t id = (int32_t)__ldg(&b.leaf_id[list[base + k]]);
+                if (t < tm || (t == tm && best >= 0 && id < best)) {
+                    tm = t;
+                    best = id;
+                }
             }
         }
     }

@@ -123,20 +123,19 @@ __device__ __forceinline__ float4 light_dir(const SceneView& sc, uint32_t li, fl
 // nodes are popped at a time and their 32 slots tested one per lane (a node a
 // step left 28 lanes idle, and a warp's walk a chain of every node it visits:
 // the lists of a 3840x2160 view of 65,536 spheres took 1,230 + 1,070 us, now
-// 450 + 350); a leaf cluster's spheres get the sphere test the brute-force masks
+// 370 + 270); a leaf cluster's spheres get the sphere test the brute-force masks
 // use, one per lane, two clusters of up to 16 at once.  All lanes call it with
-// the warp's own stack in shared memory.  Adds the candidates to the count of
-// those found before (the first cap of them written to out when FILL) and
-// returns it, or kNoTileList when the walk overflows its stack or step budget
-// or the list would pass kTileListMax.
+// the warp's own stack in shared memory.  Returns the number of candidates
+// (written to out when FILL), or kNoTileList when the walk overflows its stack
+// or step budget or the list would pass cap.
 constexpr uint32_t kWalkStack = 128;
 
 template <bool FILL>
-__device__ uint32_t tile_walk(const BvhView& b, const WarpCone& cone, float3 o, uint32_t* stack, uint32_t count,
-                              uint32_t* out, uint32_t cap)
+__device__ uint32_t tile_walk(const BvhView& b, const WarpCone& cone, float3 o, uint32_t* stack, uint32_t* out,
+                              uint32_t cap)
 {
     const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
-    uint32_t sp = 1u;
+    uint32_t sp = 1u, count = 0u;
     uint32_t budget = 2u * b.n_leaves + 8u;
     __syncwarp();
     if (lane == 0u) stack[0] = b.root;
@@ -187,57 +186,77 @@ __device__ uint32_t tile_walk(const BvhView& b, const WarpCone& cone, float3 o, 
                 meets = cone_meets(cone, mk3(s.x - o.x, s.y - o.y, s.z - o.z), cone_radius(s.w), 0.0f, 0.0f);
             }
             const uint32_t bits = __ballot_sync(kFull, meets);
-            if (count + (uint32_t)__popc(bits) > kTileListMax) return kNoTileList;
-            const uint32_t at = count + (uint32_t)__popc(bits & below);
-            if (FILL && meets && at < cap) out[at] = first + q;
+            if (count + (uint32_t)__popc(bits) > cap) return kNoTileList;
+            if (FILL && meets) out[count + (uint32_t)__popc(bits & below)] = first + q;
             count += (uint32_t)__popc(bits);
         }
     }
     return count;
 }
 
-// Primary nearest hit once per pixel of the wave (shared by its samples).
-// A warp's 32 neighbouring primary rays share the camera as apex and a narrow
-// cone of directions, so the candidates are found once per warp:
+// Pixel of lane `lane` in tile t of an image `width` across.
+__device__ __forceinline__ uint32_t tile_pixel(uint32_t t, uint32_t lane, uint32_t width, uint32_t height, bool& in)
+{
+    const uint32_t across = tiles_across(width);
+    const uint32_t x = t % across * kTileW + lane % kTileW, y = t / across * kTileH + lane / kTileW;
+    in = x < width && y < height;
+    return y * width + x;
+}
+
+// Primary nearest hit once per pixel of the wave (shared by its samples), a
+// warp to a tile (the wave's pixels of it).  The tile's primary rays share the
+// camera as apex and a narrow cone of directions, so the candidates are found
+// once per warp:
 //   the camera's tile mask or candidate list where it has them (a camera that
-//   stayed put) and the warp's pixels are one tile;
+//   stayed put);
 //   else, on the brute-force tables, every sphere's cap (worked out by the
 //   block beforehand, cone_cap) against the warp's cone: 15 instructions
 //   a sphere against 45 when each warp works the caps out itself (k_primary of
-//   1920x1080 pixels with 256 spheres 59 -> 40 us);
+//   1920x1080 pixels with 256 spheres 59 -> 38 us);
 //   else, on the LBVH, a walk of the warp's cone into a list in shared memory.
 //   The rays' own walks pay for the same nodes 32 times over, diverging
-//   (3840x2160 pixels over 65,536 spheres: 16.3 -> 1.25 ms); they remain for
-//   warps without a cone or with more candidates than the list holds.
+//   (3840x2160 pixels over 65,536 spheres: 16.3 -> 0.71 ms; 1280x720 over 4,096
+//   spread and 40,000 clustered ones 151 -> 67 and 230 -> 126 us).  They remain
+//   for warps whose list would overflow, and for images of fewer than two
+//   pixels a sphere, where a tile's cone meets so many that most lists do
+//   (287x175 pixels over 40,000 clustered spheres: 146 against 186 us).
 // With per-(pixel, light) shadow rays (wave_light_vis) it also clears the
 // pixel's visibility word, stores at the pixel's hit slot the hit point with
 // its sphere and the shadow-ray origin with the pixel, and queues in q[0], as
 // bounce 0's shadow rays, one entry (hit slot, light) per distinct light the
 // pixel's samples pick (q[0] is idle until the second bounce).
 constexpr uint32_t kCapSpheres = kTileMaskMaxSpheres;   // caps a block keeps (24 B each)
-constexpr uint32_t kWalkList = 512;                     // candidates a warp's walk keeps (2 KB)
+constexpr uint32_t kWalkList = kTileListMax;            // candidates a warp's walk keeps before it gives up (4 KB)
 
 template <int IS>
 __global__ void __launch_bounds__(kThreads) k_primary(SceneView sc, CameraView cam, WaveState ws, WaveJob job)
 {
     extern __shared__ float4 s_dyn[];   // caps, or a candidate list per warp (primary_smem)
     const uint32_t n = job.n_pixels;
-    if (blockIdx.x * blockDim.x >= n) return;
+    // the tiles of the wave's rows of pixels
+    const uint32_t across = tiles_across(cam.width);
+    const uint32_t band0 = job.pixel0 / cam.width / kTileH, band1 = (job.pixel0 + n - 1u) / cam.width / kTileH;
+    const uint32_t first = band0 * across, last = (band1 + 1u) * across, warps = blockDim.x / 32u;
+    if (first + blockIdx.x * warps >= last) return;
     const bool cached = job.prim_cached != 0;   // uniform: only the hit queue is built
     const float3 o = mk3(cam.pos[0], cam.pos[1], cam.pos[2]);
     const bool caps = IS != kIsBvh && !cached && !cam.masks && sc.n_sph <= kCapSpheres;   // uniform
     float2* cap2 = reinterpret_cast<float2*>(s_dyn + sc.n_sph);
     if (caps) stage_caps(sc.sph, sc.n_sph, o, s_dyn, cap2);
-    const bool walk = IS == kIsBvh && !cached && !cam.tile_info && sc.bvh.n_leaves > sc.bvh.leaf_size;   // uniform
+    __shared__ float4 s_stage[IS == kIsBvh ? kThreads : 1];
+    float4* stage = s_stage + (IS == kIsBvh ? threadIdx.x & ~31u : 0u);   // LBVH: this warp's 32
+    const bool walk = IS == kIsBvh && !cached && !cam.tile_info && sc.bvh.n_leaves > sc.bvh.leaf_size &&
+                      2u * (uint64_t)sc.n_sph <= (uint64_t)cam.width * cam.height;   // uniform
     uint32_t* list = reinterpret_cast<uint32_t*>(s_dyn) + (threadIdx.x >> 5) * (kWalkList + kWalkStack);
-    const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t* hits = &ws.counters[2 * ((uint32_t)job.max_bounces + 1u)];
     uint2* prim = job.prim_cache ? job.prim_cache + job.pixel0 : ws.prim;
     const bool vis = wave_light_vis(job, sc.n_lights);   // uniform
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {   // warp-uniform trip count
-        const uint32_t j = base + threadIdx.x;
-        const bool me = j < n;
-        const uint32_t p = job.pixel0 + j;
+    for (uint32_t tile = first + blockIdx.x * warps + threadIdx.x / 32u; tile < last; tile += gridDim.x * warps) {
+        bool me;
+        const uint32_t p = tile_pixel(tile, lane_id(), cam.width, cam.height, me);
+        const uint32_t j = p - job.pixel0;
+        me = me && p >= job.pixel0 && j < n;
+        if (!__any_sync(kFull, me)) continue;
         int32_t id = -1;
         float t = 0.0f;
         float3 d = o;
@@ -250,56 +269,31 @@ __global__ void __launch_bounds__(kThreads) k_primary(SceneView sc, CameraView c
             }
         } else {
             if (me) d = primary_ray(cam, p);
-            // a warp whose pixels are one aligned tile (its first pixel inside
-            // the wave, so the tile is inside the image) takes the camera's
-            // tile mask or candidate list
-            const uint32_t warp_j = base + (threadIdx.x & ~31u);                  // warp-uniform
-            const uint32_t tile_px = job.pixel0 + warp_j;
-            const bool tiled = warp_j < n && (tile_px & 31u) == 0u;
             WarpCone cone;
-            if (IS != kIsBvh && cam.masks && tiled) {
-                id = nearest_masked(sc.sph, cam.masks + (size_t)(tile_px >> 5) * cam.mask_words, cam.mask_words, o, d,
-                                    me, t);
-            } else if (IS != kIsBvh && warp_j < n) {
-                bool first;
-                const uint32_t groups = row_groups(me, p, cam.width, first);
-                for (uint32_t g = 0; g < groups; ++g) {
-                    const bool in = me && first == (g == 0u);
-                    float tg = 0.0f;
-                    int32_t h = -1;
-                    if (!warp_cone(in, d, cone)) {
-                        if (in) h = nearest_brute<false>(sc.sph, sc.n_sph, o, d, tg);
-                    } else if (caps) {
-                        h = nearest_caps(sc.sph, sc.n_sph, s_dyn, cap2, o, d, in, cone, tg);
-                    } else {
-                        h = nearest_cone(sc.sph, sc.n_sph, o, d, in, cone, tg);
-                    }
-                    if (in) id = h, t = tg;
-                }
-            } else if (IS == kIsBvh && warp_j < n) {
+            if (IS == kIsBvh) {
                 uint2 ti = make_uint2(0u, kNoTileList);
                 const uint32_t* from = list;
-                if (walk) {
-                    bool first;
-                    const uint32_t groups = row_groups(me, p, cam.width, first);
-                    ti.y = 0u;
-                    for (uint32_t g = 0; g < groups && ti.y != kNoTileList; ++g) {
-                        if (warp_cone(me && first == (g == 0u), d, cone))
-                            ti.y = tile_walk<true>(sc.bvh, cone, o, list + kWalkList, ti.y, list, kWalkList);
-                        else ti.y = kNoTileList;
-                        if (ti.y > kWalkList) ti.y = kNoTileList;
-                    }
-                    __syncwarp();   // the list is written
-                } else if (cam.tile_info && tiled) {
-                    ti = __ldg(&cam.tile_info[tile_px >> 5]);
+                if (cam.tile_info) {
+                    ti = __ldg(&cam.tile_info[tile]);
                     from = cam.tile_lists + ti.x;
+                } else if (walk && warp_cone(me, d, cone)) {
+                    ti.y = tile_walk<true>(sc.bvh, cone, o, list + kWalkList, list, kWalkList);
+                    __syncwarp();   // the list is written
                 }
                 if (ti.y != kNoTileList) {
-                    id = nearest_listed(sc.bvh, from, ti.y, o, d, me, t);
+                    id = nearest_listed(sc.bvh, from, ti.y, o, d, me, stage, t);
                     if (walk) __syncwarp();   // read before the next tile's walk writes it
                 } else if (me) {
                     id = bvh_nearest(sc.bvh, o, d, t);
                 }
+            } else if (cam.masks) {
+                id = nearest_masked(sc.sph, cam.masks + (size_t)tile * cam.mask_words, cam.mask_words, o, d, me, t);
+            } else if (!warp_cone(me, d, cone)) {
+                if (me) id = nearest_brute<false>(sc.sph, sc.n_sph, o, d, t);
+            } else if (caps) {
+                id = nearest_caps(sc.sph, sc.n_sph, s_dyn, cap2, o, d, me, cone, t);
+            } else {
+                id = nearest_cone(sc.sph, sc.n_sph, o, d, me, cone, t);
             }
             if (me) prim[j] = make_uint2(__float_as_uint(t), (uint32_t)id);
         }
@@ -1173,76 +1167,67 @@ __global__ void k_dir_table(CameraView cam, float4* out)
     }
 }
 
-// Tile masks (CameraView::masks): one warp per tile of 32 pixels builds the
-// cones of their primary directions as k_primary does (row_groups, warp_cone
-// over the same directions, primary_ray) and sets bit i where sphere i's cap
-// meets one of them, or every bit when a cone is too wide.  A
-// k_primary warp whose pixels are this tile, or part of it, has its directions
-// inside these cones.
+// Tile masks (CameraView::masks): one warp per tile builds the cone of its
+// pixels' primary directions as k_primary does (warp_cone over the same
+// directions, primary_ray) and sets bit i where sphere i's cap meets it, or
+// every bit when the cone is too wide.  A k_primary warp with part of the
+// tile's pixels has its directions inside this cone.
 __global__ void __launch_bounds__(kThreads) k_tile_masks(SceneView sc, CameraView cam, uint32_t* masks)
 {
-    const uint64_t px = (uint64_t)cam.width * cam.height;
-    const uint64_t tiles = (px + 31u) / 32u;
+    const uint32_t tiles = (uint32_t)tile_count(cam.width, cam.height);
     const uint32_t words = tile_mask_words(sc.n_sph);
     const uint32_t lane = threadIdx.x & 31u;
     const float3 o = mk3(cam.pos[0], cam.pos[1], cam.pos[2]);
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32u);
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
     extern __shared__ float4 s_dyn[];   // caps, as k_primary's
     float2* cap2 = reinterpret_cast<float2*>(s_dyn + sc.n_sph);
     stage_caps(sc.sph, sc.n_sph, o, s_dyn, cap2);
-    for (uint64_t t = (uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u; t < tiles; t += warps) {
-        const uint64_t p = 32u * t + lane;
-        const bool me = p < px;
+    for (uint32_t t = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u; t < tiles; t += warps) {
+        bool me;
+        const uint32_t p = tile_pixel(t, lane, cam.width, cam.height, me);
         float3 d = o;
-        if (me) d = primary_ray(cam, (uint32_t)p);
-        bool first;
-        const uint32_t groups = row_groups(me, (uint32_t)p, cam.width, first);
-        for (uint32_t g = 0; g < groups; ++g) {
-            WarpCone cone;
-            const bool ok = warp_cone(me && first == (g == 0u), d, cone);
-            for (uint32_t w = 0; w < words; ++w) {
-                const uint32_t i = 32u * w + lane;
-                const bool pass = i < sc.n_sph && (!ok || cap_in_cone(s_dyn[i], cap2[i], cone));
-                const uint32_t bits = __ballot_sync(kFull, pass);
-                if (lane == 0u) masks[t * words + w] = g ? masks[t * words + w] | bits : bits;
-            }
+        if (me) d = primary_ray(cam, p);
+        WarpCone cone;
+        const bool ok = warp_cone(me, d, cone);
+        for (uint32_t w = 0; w < words; ++w) {
+            const uint32_t i = 32u * w + lane;
+            const bool pass = i < sc.n_sph && (!ok || cap_in_cone(s_dyn[i], cap2[i], cone));
+            const uint32_t bits = __ballot_sync(kFull, pass);
+            if (lane == 0u) masks[(size_t)t * words + w] = bits;
         }
     }
 }
 
-// One warp per tile: the cones of the tile's primary directions (as k_primary
-// and k_tile_masks build them) and their candidate walks.  FILL: only tiles with a
+// One warp per tile: the cone of the tile's primary directions (as k_primary
+// and k_tile_masks build it) and its candidate walk.  FILL: only tiles with a
 // list, written from lists + info[t].x.
 template <bool FILL>
 __global__ void __launch_bounds__(kThreads) k_tile_lists(SceneView sc, CameraView cam, uint2* info, uint32_t* lists)
 {
-    const uint64_t px = (uint64_t)cam.width * cam.height;
-    const uint64_t tiles = (px + 31u) / 32u;
+    const uint32_t tiles = (uint32_t)tile_count(cam.width, cam.height);
     const uint32_t lane = lane_id();
     const float3 o = mk3(cam.pos[0], cam.pos[1], cam.pos[2]);
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32u);
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
     __shared__ uint32_t stacks[kThreads / 32][kWalkStack];
-    for (uint64_t t = (uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u; t < tiles; t += warps) {
+    uint32_t* stack = stacks[threadIdx.x / 32u];
+    for (uint32_t t = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u; t < tiles; t += warps) {
         uint2 ti = make_uint2(0u, 0u);
         if (FILL) {
             ti = info[t];
             if (ti.y == kNoTileList || ti.y == 0u) continue;   // warp-uniform
         }
-        const uint64_t p = 32u * t + lane;
-        const bool me = p < px;
+        bool me;
+        const uint32_t p = tile_pixel(t, lane, cam.width, cam.height, me);
         float3 d = o;
-        if (me) d = primary_ray(cam, (uint32_t)p);
-        bool first;
-        const uint32_t groups = row_groups(me, (uint32_t)p, cam.width, first);
-        uint32_t len = 0u;
-        for (uint32_t g = 0; g < groups && len != kNoTileList; ++g) {
-            WarpCone cone;
-            if (warp_cone(me && first == (g == 0u), d, cone))
-                len = tile_walk<FILL>(sc.bvh, cone, o, stacks[threadIdx.x / 32u], len, FILL ? lists + ti.x : nullptr,
-                                      ti.y);
-            else len = kNoTileList;
+        if (me) d = primary_ray(cam, p);
+        WarpCone cone;
+        const bool ok = warp_cone(me, d, cone);
+        if (FILL) {
+            if (ok) tile_walk<true>(sc.bvh, cone, o, stack, lists + ti.x, ti.y);
+        } else {
+            const uint32_t len = ok ? tile_walk<false>(sc.bvh, cone, o, stack, nullptr, kTileListMax) : kNoTileList;
+            if (lane == 0u) info[t] = make_uint2(0u, len);
         }
-        if (!FILL && lane == 0u) info[t] = make_uint2(0u, len);
     }
 }
 
@@ -1506,7 +1491,7 @@ cudaError_t enqueue_tile_masks(const SceneView& sc, const CameraView& cam, uint3
 {
     const uint64_t px = (uint64_t)cam.width * cam.height;
     if (px == 0 || sc.n_sph == 0 || sc.n_sph > kTileMaskMaxSpheres) return cudaErrorInvalidValue;
-    const uint64_t tiles = (px + 31u) / 32u;
+    const uint64_t tiles = tile_count(cam.width, cam.height);
     k_tile_masks<<<grid_for(tiles * 32u, kThreads, 1024), kThreads, primary_smem(kIsGlobal, sc.n_sph, kThreads, false),
                    stream>>>(sc, cam, masks);
     return cudaGetLastError();
@@ -1517,7 +1502,7 @@ cudaError_t enqueue_tile_list_counts(const SceneView& sc, const CameraView& cam,
 {
     const uint64_t px = (uint64_t)cam.width * cam.height;
     if (px == 0 || !sc.use_bvh || sc.bvh.n_leaves < 2) return cudaErrorInvalidValue;
-    const uint64_t tiles = (px + 31u) / 32u;
+    const uint64_t tiles = tile_count(cam.width, cam.height);
     k_tile_lists<false><<<grid_for(tiles * 32u, kThreads, 4096), kThreads, 0, stream>>>(sc, cam, info, nullptr);
     k_tile_list_scan<<<1, kScanThreads, 0, stream>>>(info, tiles, total);
     return cudaGetLastError();
@@ -1528,7 +1513,7 @@ cudaError_t enqueue_tile_list_fill(const SceneView& sc, const CameraView& cam, c
 {
     const uint64_t px = (uint64_t)cam.width * cam.height;
     if (px == 0 || !sc.use_bvh || sc.bvh.n_leaves < 2) return cudaErrorInvalidValue;
-    const uint64_t tiles = (px + 31u) / 32u;
+    const uint64_t tiles = tile_count(cam.width, cam.height);
     k_tile_lists<true><<<grid_for(tiles * 32u, kThreads, 4096), kThreads, 0, stream>>>(
         sc, cam, const_cast<uint2*>(info), lists);
     return cudaGetLastError();

@@ -161,9 +161,9 @@ struct CameraView {
     // (Camera.cpp:161-195); nullptr: computed where needed.
     const float4* dirs;
     // Optional per-tile sphere masks for this camera, eye and scene
-    // (k_tile_masks): for tile t, the 32 pixels 32t..32t+31, bit i % 32 of
-    // word t * mask_words + i / 32 is set unless sphere i certainly misses
-    // every one of their primary rays.  nullptr: culled per warp when needed.
+    // (k_tile_masks): for tile t (tile_count), bit i % 32 of word
+    // t * mask_words + i / 32 is set unless sphere i certainly misses every
+    // one of its pixels' primary rays.  nullptr: culled per warp when needed.
     const uint32_t* masks;
     uint32_t mask_words;
     // Optional per-tile candidate lists for LBVH scenes (k_tile_lists), for
@@ -173,6 +173,17 @@ struct CameraView {
     const uint2* tile_info;
     const uint32_t* tile_lists;
 };
+
+// Tiles: 8 x 4 pixels of the image, row by row of tiles; a warp traces the
+// primary rays of one.  A row of 32 pixels would be a cone 3.6 times as wide,
+// with the candidates of that cone's whole circle (and as wide as the image
+// where a warp's pixels end one row and start the next).
+constexpr uint32_t kTileW = 8, kTileH = 4;
+__host__ __device__ inline uint32_t tiles_across(uint32_t width) { return (width + kTileW - 1u) / kTileW; }
+__host__ __device__ inline uint64_t tile_count(uint32_t width, uint32_t height)
+{
+    return (uint64_t)tiles_across(width) * ((height + kTileH - 1u) / kTileH);
+}
 
 constexpr uint32_t kNoTileList = 0xffffffffu;
 constexpr uint32_t kTileListMax = 1024;   // longer lists are not kept (the rays walk the LBVH)
@@ -307,7 +318,7 @@ cudaError_t enqueue_primary_dirs(const CameraView& cam, float* out, cudaStream_t
 cudaError_t enqueue_dir_table(const CameraView& cam, float4* out, cudaStream_t stream);
 
 // Tile masks (see CameraView::masks) for scenes on the brute-force tables with
-// at most kTileMaskMaxSpheres spheres: ceil(W*H/32) * ceil(n/32) words.
+// at most kTileMaskMaxSpheres spheres: tile_count(W, H) * ceil(n/32) words.
 constexpr uint32_t kTileMaskMaxSpheres = 1024;
 __host__ __device__ inline uint32_t tile_mask_words(uint32_t n_sph) { return (n_sph + 31u) / 32u; }
 cudaError_t enqueue_tile_masks(const SceneView& sc, const CameraView& cam, uint32_t* masks, cudaStream_t stream);
