@@ -132,38 +132,44 @@ __device__ __forceinline__ void ray_hit(float4 sph, float3 o, float3 d, float t,
 // (den >= pi a2^2, g >= 1/8, denom >= 0.001), so the regrouping changes X by
 // a few units in the last place; the diffuse term's / pi is * (1 / pi).
 
-__device__ __forceinline__ float3 cook_torrance(float3 albedo, float3 f0, float metallic, float rough, float3 n,
-                                                float3 v, float3 l)
+// A material as the shading uses it (DevMaterial, make_material): what only
+// depends on the material is worked out once at upload.
+struct Brdf {
+    float3 albedo, base, emission;   // base = mix(F0, albedo, metallic)
+    float omm, a2, k;                // 1 - metallic, roughness^4, (roughness + 1)^2 / 8
+    bool metal, emits;
+};
+
+__device__ __forceinline__ float n_dot_v(float3 n, float3 v) { return gmax(dot3(n, v), 1e-7f); }
+
+// ndotv = n_dot_v(n, v).
+__device__ __forceinline__ float3 cook_torrance(const Brdf& m, float3 n, float3 v, float ndotv, float3 l)
 {
     float3 h = normalize3(add3(v, l));
     float ndotl = gmax(dot3(n, l), 1e-7f);
-    float ndotv = gmax(dot3(n, v), 1e-7f);
     float ndoth = gmax(dot3(n, h), 0.0f);
     float vdoth = gmax(dot3(v, h), 0.0f);
 
     float ct = gmin(gmax(vdoth, 0.0f), 1.0f);
-    float m = 1.0f - ct;
-    float m2 = m * m;
+    float mm = 1.0f - ct;
+    float m2 = mm * mm;
     float m4 = m2 * m2;
-    float p5 = m4 * m;
+    float p5 = m4 * mm;
+    const float3 f0 = m.base;
     float3 F = mk3(f0.x + (1.0f - f0.x) * p5, f0.y + (1.0f - f0.y) * p5, f0.z + (1.0f - f0.z) * p5);
 
-    const float a = rough * rough;
-    const float a2 = a * a;
     float nh2 = ndoth * ndoth;
-    float den = nh2 * (a2 - 1.0f) + 1.0f;
+    float den = nh2 * (m.a2 - 1.0f) + 1.0f;
     den = kPi * den * den;
-    const float r = rough + 1.0f;
-    const float k = (r * r) * 0.125f;
-    const float gv = ndotv * (1.0f - k) + k;
-    const float gl = ndotl * (1.0f - k) + k;
+    const float gv = ndotv * (1.0f - m.k) + m.k;
+    const float gl = ndotl * (1.0f - m.k) + m.k;
     float denom = 4.0f * ndotl * ndotv + 0.001f;
-    const float X = ((a2 * ndotv) * ndotl) / (((den * gv) * gl) * denom);
+    const float X = ((m.a2 * ndotv) * ndotl) / (((den * gv) * gl) * denom);
 
     float3 one_f = sub3(mk3(1.0f, 1.0f, 1.0f), F);
-    float3 kd = muls3(one_f, 1.0f - metallic);
+    float3 kd = muls3(one_f, m.omm);
     float3 spec = muls3(F, X);
-    float3 diffuse = muls3(mul3(one_f, albedo), kInvPi);
+    float3 diffuse = muls3(mul3(one_f, m.albedo), kInvPi);
     return muls3(add3(mul3(kd, diffuse), spec), ndotl);
 }
 
@@ -182,51 +188,19 @@ __device__ __forceinline__ float3 to_world(float x, float y, float z, float3 t, 
     return add3(add3(muls3(t, x), muls3(b, y)), muls3(n, z));
 }
 
-// BRDF.cu:72-93
-__device__ __forceinline__ float3 sample_cosine(float3 n, uint32_t& seed)
-{
-    const float u1 = pcg_float(seed);
-    const float u2 = pcg_float(seed);
-    const float r = sqrtf(u1);
-    float c, s;
-    sincos_2pi(u2, c, s);
-    const float x = r * c;
-    const float y = r * s;
-    const float z = sqrtf(1.0f - u1);
-    float3 t, b;
-    tangent_frame(n, t, b);
-    return to_world(x, y, z, t, b, n);
-}
-
-// BRDF.cu:95-117: the sampled half vector is returned as the new direction.
-__device__ __forceinline__ float3 sample_ggx(float3 n, float rough, uint32_t& seed)
-{
-    const float u1 = pcg_float(seed);
-    const float u2 = pcg_float(seed);
-    const float a = rough * rough;
-    const float cos_t = sqrtf((1.0f - u1) / (1.0f + (a * a - 1.0f) * u1));
-    const float sin_t = sqrtf(1.0f - cos_t * cos_t);
-    float c, s;
-    sincos_2pi(u2, c, s);
-    float3 t, b;
-    tangent_frame(n, t, b);
-    return to_world(sin_t * c, sin_t * s, cos_t, t, b, n);
-}
-
-// Renderer.cu:381-384: the next direction, sample_ggx for a metallic surface
-// and sample_cosine otherwise, with their shared steps written once: only the
-// polar terms differ (GGX: sin and cos of the sampled half-vector angle;
+// Renderer.cu:381-384: the next direction in the tangent frame (t, b, n),
+// BRDF.cu:95-117 (the sampled GGX half vector) for a metallic surface and
+// BRDF.cu:72-93 (cosine) otherwise, with their shared steps written once: only
+// the polar terms differ (GGX: sin and cos of the sampled half-vector angle;
 // cosine: sqrt(u1) and sqrt(1 - u1)), so a warp whose lanes take both kinds
-// runs the random numbers, the sin/cos of 2*pi*u2, the tangent frame and the
-// change of basis once.  Every value is computed as in the two functions.
-__device__ __forceinline__ float3 sample_next(float3 n, float rough, float metallic, uint32_t& seed)
+// runs the random numbers, the sin/cos of 2*pi*u2 and the change of basis once.
+__device__ __forceinline__ float3 sample_next(const Brdf& m, float3 t, float3 b, float3 n, uint32_t& seed)
 {
     const float u1 = pcg_float(seed);
     const float u2 = pcg_float(seed);
     float radial, z;
-    if (metallic > 0.0f) {
-        const float a = rough * rough;
-        const float cos_t = sqrtf((1.0f - u1) / (1.0f + (a * a - 1.0f) * u1));
+    if (m.metal) {
+        const float cos_t = sqrtf((1.0f - u1) / (1.0f + (m.a2 - 1.0f) * u1));
         radial = sqrtf(1.0f - cos_t * cos_t);
         z = cos_t;
     } else {
@@ -235,8 +209,6 @@ __device__ __forceinline__ float3 sample_next(float3 n, float rough, float metal
     }
     float c, s;
     sincos_2pi(u2, c, s);
-    float3 t, b;
-    tangent_frame(n, t, b);
     return to_world(radial * c, radial * s, z, t, b, n);
 }
 

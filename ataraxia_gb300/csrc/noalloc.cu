@@ -58,18 +58,9 @@ __global__ void k_convert(const atx_sphere* s, uint32_t n, const atx_material* m
         sph[i] = make_float4(s[i].center[0], s[i].center[1], s[i].center[2], r * r);
         smat[i] = ((uint32_t)s[i].material >= nm) ? 0 : s[i].material;   // Renderer.cu:30-37
     }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nm; i += stride) {
-        DevMaterial d;
-        for (int k = 0; k < 3; ++k) {
-            d.albedo[k] = m[i].albedo[k];
-            d.f0[k] = m[i].f0[k];
-            d.emission[k] = m[i].emission_color[k] * m[i].emission_intensity;
-        }
-        d.roughness = m[i].roughness;
-        d.metallic = m[i].metallic;
-        d.emission_intensity = m[i].emission_intensity;
-        mat[i] = d;
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nm; i += stride)
+        mat[i] = make_material(m[i].albedo, m[i].roughness, m[i].metallic, m[i].f0, m[i].emission_color,
+                               m[i].emission_intensity);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += stride) {
         DevLight d;
         for (int k = 0; k < 3; ++k) {

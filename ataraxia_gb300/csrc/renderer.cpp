@@ -43,17 +43,9 @@ atx_status SceneStore::upload(const atx_sphere* s, uint32_t n, const atx_materia
         srad[i] = r;
     }
     std::vector<DevMaterial> mats(nm);
-    for (uint32_t i = 0; i < nm; ++i) {
-        DevMaterial& d = mats[i];
-        for (int k = 0; k < 3; ++k) {
-            d.albedo[k] = m[i].albedo[k];
-            d.f0[k] = m[i].f0[k];
-            d.emission[k] = m[i].emission_color[k] * m[i].emission_intensity;  // Scene.h:41
-        }
-        d.roughness = m[i].roughness;
-        d.metallic = m[i].metallic;
-        d.emission_intensity = m[i].emission_intensity;
-    }
+    for (uint32_t i = 0; i < nm; ++i)
+        mats[i] = make_material(m[i].albedo, m[i].roughness, m[i].metallic, m[i].f0, m[i].emission_color,
+                                m[i].emission_intensity);
     std::vector<DevLight> lts(nl);
     for (uint32_t i = 0; i < nl; ++i) {
         for (int k = 0; k < 3; ++k) {

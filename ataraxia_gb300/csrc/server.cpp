@@ -292,7 +292,7 @@ double Server::now() const
 uint64_t Server::job_bytes(const atx_batch_scene& s, uint32_t bvh_threshold)
 {
     const uint64_t n = s.n_spheres;
-    uint64_t b = up256(16 * n) + up256(4 * n) + up256(4 * n) + up256(48ull * s.n_materials) + up256(32ull * s.n_lights);
+    uint64_t b = up256(16 * n) + up256(4 * n) + up256(4 * n) + up256(sizeof(DevMaterial) * (uint64_t)s.n_materials) + up256(32ull * s.n_lights);
     const bool bvh = n >= (bvh_threshold ? bvh_threshold : kDefaultBvhThreshold) && n > 1;
     if (bvh) b += up256(lbvh_bytes((uint32_t)n));
     // light and direction buffers, as SceneStore::upload builds them

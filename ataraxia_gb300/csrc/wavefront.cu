@@ -194,6 +194,51 @@ __device__ uint32_t tile_walk(const BvhView& b, const WarpCone& cone, float3 o, 
     return count;
 }
 
+// What the samples of a hit pixel share at the first bounce (per-(pixel, light)
+// shadow rays only), computed once per pixel by k_primary and read by all its
+// samples: hit point, normal and tangent frame, shadow and continuation origin,
+// view direction.  Two float4 rows per hit slot in each of sh_o, sh_d and sh_c,
+// which are idle until then (a wave with several samples per pixel has at least
+// two path slots per pixel).
+struct PixelRecord {
+    float3 pos, nrm, so, tx, ty, v;
+    float ndotv;
+    uint32_t hit, mat, j, own, p;   // sphere, material, wave pixel, sphere with a direction buffer (~0u), pixel
+};
+
+__device__ __forceinline__ float4 row4(float3 a, uint32_t w) { return make_float4(a.x, a.y, a.z, __uint_as_float(w)); }
+
+__device__ __forceinline__ void store_record(const WaveState& ws, uint32_t slot, const PixelRecord& r)
+{
+    ws.sh_o[2u * slot] = row4(r.pos, r.hit);
+    ws.sh_o[2u * slot + 1u] = row4(r.nrm, r.mat);
+    ws.sh_d[2u * slot] = row4(r.so, r.j);
+    ws.sh_d[2u * slot + 1u] = row4(r.tx, r.own);
+    ws.sh_c[2u * slot] = make_float4(r.v.x, r.v.y, r.v.z, r.ndotv);
+    ws.sh_c[2u * slot + 1u] = row4(r.ty, r.p);
+}
+
+__device__ __forceinline__ PixelRecord load_record(const WaveState& ws, uint32_t slot)
+{
+    const float4 a = ws.sh_o[2u * slot], b = ws.sh_o[2u * slot + 1u];
+    const float4 c = ws.sh_d[2u * slot], e = ws.sh_d[2u * slot + 1u];
+    const float4 f = ws.sh_c[2u * slot], g = ws.sh_c[2u * slot + 1u];
+    PixelRecord r;
+    r.pos = mk3(a.x, a.y, a.z);
+    r.hit = __float_as_uint(a.w);
+    r.nrm = mk3(b.x, b.y, b.z);
+    r.mat = __float_as_uint(b.w);
+    r.so = mk3(c.x, c.y, c.z);
+    r.j = __float_as_uint(c.w);
+    r.tx = mk3(e.x, e.y, e.z);
+    r.own = __float_as_uint(e.w);
+    r.v = mk3(f.x, f.y, f.z);
+    r.ndotv = f.w;
+    r.ty = mk3(g.x, g.y, g.z);
+    r.p = __float_as_uint(g.w);
+    return r;
+}
+
 // Pixel of lane `lane` in tile t of an image `width` across.
 __device__ __forceinline__ uint32_t tile_pixel(uint32_t t, uint32_t lane, uint32_t width, uint32_t height, bool& in)
 {
@@ -221,15 +266,17 @@ __device__ __forceinline__ uint32_t tile_pixel(uint32_t t, uint32_t lane, uint32
 //   pixels a sphere, where a tile's cone meets so many that most lists do
 //   (287x175 pixels over 40,000 clustered spheres: 146 against 186 us).
 // With per-(pixel, light) shadow rays (wave_light_vis) it also clears the
-// pixel's visibility word, stores at the pixel's hit slot the hit point with
-// its sphere and the shadow-ray origin with the pixel, and queues in q[0], as
+// pixel's visibility word, stores the pixel's record at its hit slot
+// (PixelRecord), and queues in q[0], as
 // bounce 0's shadow rays, one entry (hit slot, light) per distinct light the
 // pixel's samples pick (q[0] is idle until the second bounce).
 constexpr uint32_t kCapSpheres = kTileMaskMaxSpheres;   // caps a block keeps (24 B each)
 constexpr uint32_t kWalkList = kTileListMax;            // candidates a warp's walk keeps before it gives up (4 KB)
 
+// Four blocks per SM for the LBVH's walks (64 registers; 72 and three blocks:
+// 43 -> 57 us a lane of the 65,536-sphere scene).
 template <int IS>
-__global__ void __launch_bounds__(kThreads) k_primary(SceneView sc, CameraView cam, WaveState ws, WaveJob job)
+__global__ void __launch_bounds__(kThreads, IS == kIsBvh ? 4 : 5) k_primary(SceneView sc, CameraView cam, WaveState ws, WaveJob job)
 {
     extern __shared__ float4 s_dyn[];   // caps, or a candidate list per warp (primary_smem)
     const uint32_t n = job.n_pixels;
@@ -311,9 +358,19 @@ __global__ void __launch_bounds__(kThreads) k_primary(SceneView sc, CameraView c
         }
         if (me) ws.vis[j] = 0u;
         if (id >= 0) {
-            const float3 so = add3(pos, muls3(nrm, kOffset));
-            ws.sh_o[slot] = make_float4(pos.x, pos.y, pos.z, __uint_as_float((uint32_t)id));
-            ws.sh_d[slot] = make_float4(so.x, so.y, so.z, __uint_as_float(j));
+            PixelRecord r;
+            r.pos = pos;
+            r.hit = (uint32_t)id;
+            r.nrm = nrm;
+            r.mat = (uint32_t)__ldg(&sc.sph_mat[id]);
+            r.so = add3(pos, muls3(nrm, kOffset));
+            r.j = j;
+            tangent_frame(nrm, r.tx, r.ty);
+            r.own = db_reaches(sc, (uint32_t)id, __ldg(&sc.sph[id]), r.so) ? (uint32_t)id : ~0u;
+            r.v = neg3(d);
+            r.ndotv = n_dot_v(nrm, r.v);
+            r.p = p;
+            store_record(ws, slot, r);
         }
         // one slot range per warp, lane after lane: an inclusive scan of the
         // lanes' light counts and one atomicAdd
@@ -336,6 +393,23 @@ __global__ void __launch_bounds__(kThreads) k_primary(SceneView sc, CameraView c
     }
 }
 
+// Material mi's rows (all but the first bounce's).
+__device__ __forceinline__ Brdf load_mat(const SceneView& sc, int32_t mi)
+{
+    const float4* row = reinterpret_cast<const float4*>(sc.mat + mi);
+    const float4 m0 = __ldg(row), m1 = __ldg(row + 1), m2 = __ldg(row + 2);
+    Brdf b;
+    b.albedo = mk3(m0.x, m0.y, m0.z);
+    b.a2 = fabsf(m0.w);
+    b.metal = __float_as_int(m0.w) < 0;
+    b.base = mk3(m1.x, m1.y, m1.z);
+    b.omm = m1.w;
+    b.emission = mk3(m2.x, m2.y, m2.z);
+    b.k = fabsf(m2.w);
+    b.emits = __float_as_int(m2.w) < 0;
+    return b;
+}
+
 // What shading a hit leaves behind (Renderer.cu:318-384 for one bounce).
 struct Shaded {
     float3 add;        // emission (Renderer.cu:329-333), when touch
@@ -349,44 +423,34 @@ struct Shaded {
 
 // Shading of the hit (sphere hit at tmin) of path pid's ray (o, d) with
 // throughput thr at bounce `bounce` (seed already advanced by it): emission,
-// the light pick and its BRDF term, the shadow ray (visibility bit j for vis,
-// tested here through the light buffer for INL, else a record for k_shadow),
+// the light pick and its BRDF term, the shadow ray (tested here through the
+// light buffer for INL, else a record for k_shadow),
 // roulette and the next direction, which replace o, d, thr, own and advance
 // seed.
 template <int IS, bool INL>
 __device__ __forceinline__ void shade_hit(const SceneView& sc, const float4* sph, const WaveState& ws, uint32_t pid,
                                           int32_t hit, float tmin, float3& o, float3& d, float3& thr, uint32_t& own,
-                                          uint32_t& seed, bool last, bool vis, uint32_t j, Shaded& r)
+                                          uint32_t& seed, bool last, Shaded& r)
 {
     const float4 s = table_sphere<IS == kIsSmem>(sph, (uint32_t)hit);
     float3 pos, nrm;
     ray_hit(s, o, d, tmin, pos, nrm);
     const int32_t mi = __ldg(&sc.sph_mat[hit]);
-    const float4* mrow = reinterpret_cast<const float4*>(sc.mat + mi);
-    const float4 m0 = __ldg(mrow), m1 = __ldg(mrow + 1), m2 = __ldg(mrow + 2);
-    const float3 albedo = mk3(m0.x, m0.y, m0.z);
-    const float rough = m0.w;
-    const float3 f0 = mk3(m1.x, m1.y, m1.z);
-    const float metallic = m1.w;
+    const Brdf m = load_mat(sc, mi);
 
-    if (m2.w > 0.0f) {  // Renderer.cu:329-333
-        r.add = mul3(mk3(m2.x, m2.y, m2.z), thr);
+    if (m.emits) {  // Renderer.cu:329-333
+        r.add = mul3(m.emission, thr);
         r.touch = true;
     }
-    // glm::mix(F0, albedo, metallic), Renderer.cu:335
-    const float3 base = add3(muls3(f0, 1.0f - metallic), muls3(albedo, metallic));
 
     if (sc.n_lights > 0u) {  // Renderer.cu:338-369
         const uint32_t li = light_pick(sc, seed);
         float3 L;
         float dist2;
         const float4 l1 = light_dir(sc, li, pos, L, dist2);
-        const float3 f = cook_torrance(albedo, base, metallic, rough, nrm, neg3(d), L);
+        const float3 f = cook_torrance(m, nrm, neg3(d), n_dot_v(nrm, neg3(d)), L);
         const float3 c = mul3(mul3(mk3(l1.x, l1.y, l1.z), f), thr);
-        if (vis) {
-            r.lit = ((ws.vis[j] >> li) & 1u) != 0u;
-            r.lc = c;
-        } else if (INL) {   // Renderer.cu:348-352
+        if (INL) {   // Renderer.cu:348-352
             const float3 so = add3(pos, muls3(nrm, kOffset));
             r.lit = sc.n_sph == 0u || !occluded_lb<IS>(sc, sph, li, so, L, dist2);
             r.lc = c;
@@ -403,12 +467,14 @@ __device__ __forceinline__ void shade_hit(const SceneView& sc, const float4* sph
     }
 
     if (!last) {  // Renderer.cu:371-384
-        thr = mul3(thr, albedo);
+        thr = mul3(thr, m.albedo);
         o = add3(pos, muls3(nrm, kOffset));
         const float p = gmax(0.1f, gmin(1.0f, length3(thr)));
         if (!(pcg_float(seed) > p)) {
             thr = mul_rcp3(thr, p);
-            d = sample_next(nrm, rough, metallic, seed);
+            float3 tx, ty;
+            tangent_frame(nrm, tx, ty);
+            d = sample_next(m, tx, ty, nrm, seed);
             // the next ray leaves this sphere (~0u: beyond the direction buffer's reach)
             own = db_reaches(sc, (uint32_t)hit, s, o) ? (uint32_t)hit : ~0u;
             r.push_next = true;
@@ -473,7 +539,11 @@ __device__ __forceinline__ void push_hit(const WaveState& ws, uint32_t* qout, ui
 // took 249 us for 1920x1080 on the 256-sphere scene against 59 + 35 us.
 // INL: the scene has a light buffer and shadow rays are tested right after
 // the shading (a lookup and a few spheres) instead of through k_shadow.
-template <int IS, bool INL>
+// REC: per-(pixel, light) shadow rays (wave_light_vis): what a pixel's samples
+// share comes from its record, the light of a sample is added here when
+// k_shadow found it visible from the pixel's hit, and throughput and roulette
+// probability after the first bounce from the material's last row.
+template <int IS, bool INL, bool REC>
 __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
     k_first(SceneView sc, CameraView cam, WaveState ws, WaveJob job)
 {
@@ -481,9 +551,6 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
     if (blockIdx.x * blockDim.x >= n) return;
     const bool last = 1 >= job.max_bounces;
     const uint32_t stride = gridDim.x * blockDim.x;
-    // per-(pixel, light) shadow rays: the light of a sample is added here when
-    // k_shadow found it visible from the pixel's hit
-    const bool vis = wave_light_vis(job, sc.n_lights);
     const uint2* prim = job.prim_cache ? job.prim_cache + job.pixel0 : ws.prim;
     uint32_t missed = 0u;   // INL: continuation rays traced here that missed
 
@@ -495,19 +562,46 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
         int32_t nhit = -1;   // INL: the next ray's hit
         float nt = 0.0f;
         if (idx < n) {
-            const uint32_t j = ws.hitq[idx / job.spp];   // path ids stay pixel-major
-            const uint32_t smp = idx % job.spp;
-            pid = j * job.spp + smp;
-            const uint32_t p = job.pixel0 + j;
-            o = mk3(cam.pos[0], cam.pos[1], cam.pos[2]);
-            d = primary_ray(cam, p);
-            thr = mk3(1.f, 1.f, 1.f);
-            seed = p * (job.frame0 + smp);   // bounce 0: seed += 0
-            const uint2 pr = prim[j];
-            shade_hit<IS, INL>(sc, sc.sph, ws, pid, (int32_t)pr.y, __uint_as_float(pr.x), o, d, thr, own, seed,
-                                  last, vis, j, r);
-            float3 c = add3(mk3(0.f, 0.f, 0.f), r.add);
-            if (r.lit) c = add3(c, r.lc);   // as k_shadow adds it: after the emission
+            const uint32_t slot = job.spp == 1u ? idx : (uint32_t)__umul64hi(job.spp_div, (uint64_t)idx);   // idx / spp
+            const uint32_t smp = idx - slot * job.spp;
+            float3 c = mk3(0.f, 0.f, 0.f);
+            if (REC) {
+                const PixelRecord px = load_record(ws, slot);
+                pid = px.j * job.spp + smp;   // path ids stay pixel-major
+                seed = px.p * (job.frame0 + smp);   // bounce 0: seed += 0
+                const Brdf m = load_mat(sc, (int32_t)px.mat);
+                if (m.emits) c = add3(c, m.emission);   // Renderer.cu:329-333, throughput (1, 1, 1)
+                const uint32_t li = light_pick(sc, seed);
+                if ((ws.vis[px.j] >> li) & 1u) {
+                    float3 L;
+                    float dist2;
+                    const float4 l1 = light_dir(sc, li, px.pos, L, dist2);
+                    c = add3(c, mul3(mk3(l1.x, l1.y, l1.z), cook_torrance(m, px.nrm, px.v, px.ndotv, L)));
+                }
+                if (!last) {   // Renderer.cu:371-384
+                    const float4 m3 = __ldg(reinterpret_cast<const float4*>(sc.mat + px.mat) + 3);
+                    if (!(pcg_float(seed) > m3.w)) {
+                        thr = mk3(m3.x, m3.y, m3.z);
+                        d = sample_next(m, px.tx, px.ty, px.nrm, seed);
+                        o = px.so;
+                        own = px.own;
+                        r.push_next = true;
+                    }
+                }
+            } else {
+                const uint32_t j = ws.hitq[slot];
+                pid = j * job.spp + smp;
+                const uint32_t p = job.pixel0 + j;
+                o = mk3(cam.pos[0], cam.pos[1], cam.pos[2]);
+                d = primary_ray(cam, p);
+                thr = mk3(1.f, 1.f, 1.f);
+                seed = p * (job.frame0 + smp);
+                const uint2 pr = prim[j];
+                shade_hit<IS, INL>(sc, sc.sph, ws, pid, (int32_t)pr.y, __uint_as_float(pr.x), o, d, thr, own, seed,
+                                   last, r);
+                c = add3(c, r.add);
+                if (r.lit) c = add3(c, r.lc);   // as k_shadow adds it: after the emission
+            }
             if (INL && r.push_next) {
                 nhit = scene_nearest_from<IS>(sc, sc.sph, own, o, d, nt);
                 r.push_next = nhit >= 0;
@@ -519,7 +613,7 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
             ws.col[pid] = make_float4(c.x, c.y, c.z, 0.0f);
         }
         if (INL) {
-            warp_push(&ws.counters[1], r.traced_sh);   // count the shadow rays tested here
+            if (!REC) warp_push(&ws.counters[1], r.traced_sh);   // count the shadow rays tested here
             push_hit(ws, ws.q[1], &ws.counters[2], r.push_next, pid, o, seed, d, nt, thr, nhit);
         } else {
             push_shaded<INL>(ws, ws.q[1], 0, pid, r, o, d, thr, own, seed);
@@ -611,7 +705,7 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
             seed = __float_as_uint(ro.w) + (uint32_t)bounce;
             d = mk3(rd.x, rd.y, rd.z);
             thr = mk3(tt.x, tt.y, tt.z);
-            shade_hit<IS, false>(sc, sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, false, 0u, r);
+            shade_hit<IS, false>(sc, sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, r);
             if (r.touch || r.lit) {
                 // emission of bounce b, then its light (the order k_shadow adds it in)
                 float4 c = ws.col[pid];
@@ -685,8 +779,7 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
             seed = __float_as_uint(ro.w) + (uint32_t)bounce;
             d = mk3(rd.x, rd.y, rd.z);
             thr = mk3(tt.x, tt.y, tt.z);
-            shade_hit<IS, true>(sc, sph, ws, pid, (int32_t)__float_as_uint(tt.w), rd.w, o, d, thr, own, seed, last,
-                                  false, 0u, r);
+            shade_hit<IS, true>(sc, sph, ws, pid, (int32_t)__float_as_uint(tt.w), rd.w, o, d, thr, own, seed, last, r);
             bool sky = false;
             if (r.push_next) {
                 nhit = scene_nearest_from<IS>(sc, sph, own, o, d, nt);
@@ -767,7 +860,7 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
             uint32_t own = ~0u;
             seed += b;
             const bool last = (int)b + 1 >= job.max_bounces;
-            shade_hit<IS, true>(sc, sc.sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, false, 0u, r);
+            shade_hit<IS, true>(sc, sc.sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, r);
             traced += r.traced_sh ? 1u : 0u;
             bool sky = false;
             if (r.push_next) {
@@ -830,7 +923,7 @@ __device__ __forceinline__ ShadowRay load_shadow(const SceneView& sc, const Wave
     if (VIS) {
         const uint32_t e = ws.q[0][idx];
         const uint32_t slot = e & kShadowSphereMask, li = e >> 26;
-        const float4 a = ws.sh_o[slot], b = ws.sh_d[slot];
+        const float4 a = ws.sh_o[2u * slot], b = ws.sh_d[2u * slot];   // PixelRecord: pos, hit; so, j
         light_dir(sc, li, mk3(a.x, a.y, a.z), r.d, r.dist2);
         r.o = mk3(b.x, b.y, b.z);
         r.tag = shadow_tag(__float_as_uint(a.w), li);
@@ -1069,19 +1162,14 @@ __global__ void __launch_bounds__(kThreads, kFusedBlocksPerSm) k_fused(SceneView
                 float3 pos, nrm;
                 ray_hit(sp, o, d, tmin, pos, nrm);
                 const int32_t mi = __ldg(&sc.sph_mat[hit]);
-                const float4* mrow = reinterpret_cast<const float4*>(sc.mat + mi);
-                const float4 m0 = __ldg(mrow), m1 = __ldg(mrow + 1), m2 = __ldg(mrow + 2);
-                const float3 albedo = mk3(m0.x, m0.y, m0.z);
-                const float rough = m0.w;
-                const float metallic = m1.w;
-                if (m2.w > 0.0f) c = add3(c, mul3(mk3(m2.x, m2.y, m2.z), thr));   // Renderer.cu:329-333
-                const float3 base = add3(muls3(mk3(m1.x, m1.y, m1.z), 1.0f - metallic), muls3(albedo, metallic));
+                const Brdf m = load_mat(sc, mi);
+                if (m.emits) c = add3(c, mul3(m.emission, thr));   // Renderer.cu:329-333
                 if (sc.n_lights > 0u) {   // Renderer.cu:338-369
                     const uint32_t li = light_pick(sc, seed);
                     float3 L;
                     float dist2;
                     const float4 l1 = light_dir(sc, li, pos, L, dist2);
-                    const float3 f = cook_torrance(albedo, base, metallic, rough, nrm, neg3(d), L);
+                    const float3 f = cook_torrance(m, nrm, neg3(d), n_dot_v(nrm, neg3(d)), L);
                     const float3 lc = mul3(mul3(mk3(l1.x, l1.y, l1.z), f), thr);
                     bool lit;
                     const uint32_t bit = 1u << (li & 31u);
@@ -1099,12 +1187,14 @@ __global__ void __launch_bounds__(kThreads, kFusedBlocksPerSm) k_fused(SceneView
                     if (lit) c = add3(c, lc);
                 }
                 if (i + 1 >= job.max_bounces) break;   // Renderer.cu:371-384 change nothing after the last
-                thr = mul3(thr, albedo);
+                thr = mul3(thr, m.albedo);
                 o = add3(pos, muls3(nrm, kOffset));
                 const float pr = gmax(0.1f, gmin(1.0f, length3(thr)));
                 if (pcg_float(seed) > pr) break;
                 thr = mul_rcp3(thr, pr);
-                d = sample_next(nrm, rough, metallic, seed);
+                float3 tx, ty;
+                tangent_frame(nrm, tx, ty);
+                d = sample_next(m, tx, ty, nrm, seed);
             }
             a.x = a.x + c.x;
             a.y = a.y + c.y;
@@ -1369,10 +1459,12 @@ cudaError_t plan_launch(const SceneView& sc, int device, int threads, LaunchShap
     return cudaSuccess;
 }
 
-cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveState& ws, const WaveJob& job,
+cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveState& ws, const WaveJob& wave,
                          const LaunchShape& shape, float4* accum, uint32_t* image, cudaStream_t stream,
                          uint32_t* launches, KernelTimer* timer)
 {
+    WaveJob job = wave;
+    job.spp_div = fastmod_multiplier(job.spp);
     uint32_t nl = 0;
     const size_t sm = shape.smem_spheres;
     const int bounces = job.max_bounces;
@@ -1417,8 +1509,9 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
             }
             begin(kFamExtend);
             constexpr int G = IS == kIsBvh ? kIsBvh : kIsGlobal;   // these read the sphere table through L1
-            if (inl) k_first<G, true><<<g0, kExtendThreads, 0, stream>>>(sc, cam, ws, job);
-            else k_first<kIsGlobal, false><<<g0, kExtendThreads, 0, stream>>>(sc, cam, ws, job);
+            const auto first = inl ? (vis ? k_first<G, true, true> : k_first<G, true, false>)
+                                   : (vis ? k_first<kIsGlobal, false, true> : k_first<kIsGlobal, false, false>);
+            first<<<g0, kExtendThreads, 0, stream>>>(sc, cam, ws, job);
             end(kFamExtend);
             ++nl;
             for (int b = 0; b < bounces; ++b) {

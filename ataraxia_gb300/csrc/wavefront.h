@@ -4,23 +4,52 @@
 // compiler can include it.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
 namespace atx {
 
-// Material as the shading code reads it: three float4 rows.  emission holds
-// emissionColor * emissionIntensity (Scene.h:41, one IEEE product done on the
-// host, the same bits the reference's getEmission() gives).
+// Material as the shading code reads it, four float4 rows (the last only at
+// the first bounce), with every value that depends on the material alone
+// worked out once (make_material), in the order the shading would: the bits
+// are the same.  emission holds emissionColor * emissionIntensity (Scene.h:41,
+// the same bits the reference's getEmission() gives).
 struct alignas(16) DevMaterial {
     float albedo[3];
-    float roughness;
-    float f0[3];
-    float metallic;
+    float a2_metal;      // roughness^4; the sign bit: metallic > 0
+    float base[3];       // mix(F0, albedo, metallic), Renderer.cu:335
+    float omm;           // 1 - metallic
     float emission[3];
-    float emission_intensity;
+    float k_emits;       // (roughness + 1)^2 / 8; the sign bit: emissionIntensity > 0
+    float thr0[3];       // throughput after the first bounce's roulette, from (1, 1, 1)
+    float p0;            // its probability, Renderer.cu:374-378
 };
-static_assert(sizeof(DevMaterial) == 48, "DevMaterial is three float4 rows");
+static_assert(sizeof(DevMaterial) == 64, "DevMaterial is four float4 rows");
+
+// Sign bits are put on squares (or NaN), which have none of their own.
+__host__ __device__ inline DevMaterial make_material(const float albedo[3], float roughness, float metallic,
+                                                     const float f0[3], const float emission_color[3],
+                                                     float emission_intensity)
+{
+    DevMaterial d;
+    const float a = roughness * roughness, a2 = a * a;
+    const float r = roughness + 1.0f;
+    for (int i = 0; i < 3; ++i) {
+        d.albedo[i] = albedo[i];
+        d.base[i] = f0[i] * (1.0f - metallic) + albedo[i] * metallic;
+        d.emission[i] = emission_color[i] * emission_intensity;
+    }
+    d.a2_metal = copysignf(a2, metallic > 0.0f ? -1.0f : 1.0f);
+    d.omm = 1.0f - metallic;
+    d.k_emits = copysignf((r * r) * 0.125f, emission_intensity > 0.0f ? -1.0f : 1.0f);
+    const float len = sqrtf(fmaf(albedo[2], albedo[2], fmaf(albedo[1], albedo[1], albedo[0] * albedo[0])));
+    const float m = len < 1.0f ? len : 1.0f;        // glm::min(1, len), glm::max(0.1, m)
+    d.p0 = 0.1f < m ? m : 0.1f;
+    const float inv = 1.0f / d.p0;
+    for (int i = 0; i < 3; ++i) d.thr0[i] = albedo[i] * inv;
+    return d;
+}
 
 // Point light: position and color * intensity (Renderer.cu:362, one product).
 struct alignas(16) DevLight {
@@ -194,6 +223,9 @@ constexpr uint32_t kTileListMax = 1024;   // longer lists are not kept (the rays
 //   q[2]   ping-pong extension queues of path ids
 //   sh_o   (shadow origin xyz, distance^2)   sh_d (direction xyz, path id bits)
 //   sh_c   (unoccluded contribution rgb, -)
+//          with per-(pixel, light) shadow rays (wave_light_vis) the three hold,
+//          until the first bounce is shaded, a record of two rows each per hit
+//          slot: what all samples of the pixel share there (PixelRecord)
 //   counters[2*b] extension rays queued for bounce b, [2*b+1] shadow rays of bounce b
 //   prim   one primary hit per pixel: the reference's primary ray depends on
 //          the pixel only (Camera.cpp:161-195, no jitter), so every sample of a
@@ -246,6 +278,7 @@ struct WaveJob {
     // holds this view's hits, so they are not traced again.
     uint2* prim_cache;
     int32_t prim_cached;
+    uint64_t spp_div;         // fastmod_multiplier(spp), set by enqueue_wave: x / spp by multiplication
 };
 
 // Whether the first bounce's shadow rays are traced once per (pixel, light)
