@@ -251,7 +251,7 @@ atx_status Batch::autotune(uint32_t passes, atx_batch_tuning* chosen)
     if (!passes) passes = 2;
     // the trials are passes over the same scenes: lists they would get on the way come first
     for (auto& p : slots_)
-        if (p && lists_ && p->scene.lists_due(2ull * kDbMaxBvhSpheres * kDbMaxBvhSpheres)) {
+        if (p && lists_ && p->scene.lists_due(16ull * kDbMaxBvhSpheres * kDbMaxBvhSpheres)) {
             p->scene.build_lists(&budget_, up_stream_);
             ATX_CUDA(cudaEventRecord(uploaded_, up_stream_));
         }

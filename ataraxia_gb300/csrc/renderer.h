@@ -39,8 +39,8 @@ struct SceneStore {
     // Light and direction buffers for an LBVH scene of up to kDbMaxBvhSpheres
     // spheres, on top of its tree.  Every pair of spheres is looked at, so they
     // are built only for a scene that goes on being rendered: lists_due counts
-    // the paths about to be traced and says when those so far would have paid
-    // for the build; a scene rendered once, or uploaded for every render, keeps
+    // the paths of each render and says, before it, when those so far would
+    // have paid for the build; a scene rendered once, or uploaded for every render, keeps
     // to the tree.  build_lists leaves the scene on the tree when a budget is
     // set, which later buffers may need in full, or when the lists would take
     // more than a quarter of the device's free memory.

@@ -43,8 +43,8 @@ def _render(sc, calls, sky, **kw):
         return out, r.stats()["device_bytes"]
 
 
-# the smallest LBVH scene, one in between and the most spheres with lists; the paths of the calls pass
-# 2 n^2 within the second call
+# the smallest LBVH scene, one in between and the most spheres with lists; the calls' paths pass
+# 2 n^2 with the second call
 @pytest.mark.parametrize("kind,n,lights,sky", [("open", 1025, 1, False), ("clump", 1300, 5, True),
                                                ("tied", 1401, 40, False), ("open", 4096, 8, False)])
 @pytest.mark.parametrize("flags", [0, _native.FLAG_OVERLAP_RENDERS])
@@ -64,9 +64,9 @@ def test_lists_wait_for_enough_paths_and_for_memory():
     frames = 2 * 1025 * 1025 // sc.pixels + 1
     _, few = _render(sc, (1, 2), False)
     assert few < 1025 * 300_000
-    want, _ = _render(sc, (1, frames), False, bvh_threshold=1 << 30)
-    with_lists, large = _render(sc, (1, frames), False)
-    got, held = _render(sc, (1, frames), False, hbm_budget_bytes=2_000_000_000)   # a budget: the tree, as before
+    want, _ = _render(sc, (1, frames, 2), False, bvh_threshold=1 << 30)
+    with_lists, large = _render(sc, (1, frames, 2), False)
+    got, held = _render(sc, (1, frames, 2), False, hbm_budget_bytes=2_000_000_000)   # a budget: the tree, as before
     assert large > held + 1025 * 300_000
     for a, b, c in zip(got, with_lists, want):
         assert bit_mismatches(a, c) == 0 and bit_mismatches(b, c) == 0
