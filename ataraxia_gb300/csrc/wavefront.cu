@@ -10,12 +10,14 @@
 //   k_bounce         bounce b >= 1 (LBVH scenes): nearest hit, then the same
 //                    shading, with the block's hits gathered in shared memory
 //                    first.
-//   With a light buffer and a direction buffer (scenes up to 1,024 spheres)
-//   shadow rays are tested right after the shading and a continuation ray is
-//   traced where it is made, so only rays that hit are queued:
-//   k_shade          bounce 1: shades its queue of hits on full warps.
-//   k_paths          bounces >= 2 in one persistent launch: each lane
+//   With a light buffer and a direction buffer (scenes up to 1,024 spheres,
+//   and LBVH scenes with cell lists) shadow rays are tested right after the
+//   shading and a continuation ray is traced where it is made, so only rays
+//   that hit are queued:
+//   k_paths          the later bounces in one persistent launch: each lane
 //                    carries a path to its end, then takes the next.
+//   k_shade          bounce 1 of LBVH scenes with such lists: shades its
+//                    queue of hits on full warps.
 //   k_shadow         any-hit over a shadow queue: the first bounce's (pixel,
 //                    light) rays, and per-sample shadow rays of LBVH scenes.
 //   k_accumulate     adds the wave's per-sample colours to the float4
@@ -46,8 +48,14 @@ constexpr int kThreads = 256;
 constexpr int kExtendThreads = 256;
 constexpr int kExtendBlocksPerSm = 4;
 // With a light buffer, bounces from this one on run in one persistent k_paths
-// launch instead of a k_bounce launch each.
-constexpr int kPathsFrom = 2;
+// launch.  On the brute-force tables every bounce after the first: against a
+// k_shade launch for bounce 1, the 1001x563 15-bounce scene takes 33.5 us
+// instead of 37.2, 256 spheres under a moving camera 229 instead of 244, 64
+// samples over 9 spheres 2.36 ms instead of 2.44.  LBVH scenes keep k_shade
+// (4,096 spheres 707 instead of 767 us): a lane that leaves its cell list for a
+// walk holds up the 31 paths of its warp, which only bounce 1's full warps hide.
+template <int IS>
+constexpr int kPathsFrom = IS == kIsBvh ? 2 : 1;
 
 // k_shadow's blocks per SM: the shared-memory variant fits 40 registers
 // without spilling (6 blocks of 256 threads); the others take up to 64 (4).
@@ -739,22 +747,16 @@ __device__ __forceinline__ float3 bounce_terms(float3 c, const Shaded& r)
     return c;
 }
 
-// Bounce b >= 1 of scenes with a light buffer: every queued ray hits (it was
+// Bounce b >= 1 of LBVH scenes with cell lists: every queued ray hits (it was
 // traced where it was made), so each thread shades one, on full warps, then
-// traces its continuation and queues it if it hits.  Launched over the
-// global sphere table (IS = kIsGlobal): the few spheres a list walk touches
-// come faster from L1 than from the shared-memory pair layout, and no block
-// stages the table.
+// traces its continuation and queues it if it hits.
 template <int IS>
 __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
     k_shade(SceneView sc, WaveState ws, WaveJob job, int bounce)
 {
-    constexpr bool SMEM = IS == kIsSmem;
-    extern __shared__ float4 s_sph[];
     const uint32_t n = ws.counters[2 * bounce];
     if (blockIdx.x * blockDim.x >= n) return;
-    if (SMEM) stage_spheres(sc, s_sph);
-    const float4* sph = SMEM ? s_sph : sc.sph;
+    const float4* sph = sc.sph;   // the few spheres a list holds come from L1
     // select, not index: a runtime index into the parameter's array would
     // copy the whole WaveState to local memory
     const uint32_t* qin = (bounce & 1) ? ws.q[1] : ws.q[0];
@@ -800,7 +802,7 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
     warp_push_n(&ws.counters[2 * ((uint32_t)job.max_bounces + 1u) + 3u], missed);
 }
 
-// The sparse late bounces (b >= b0) of scenes with a light buffer in one
+// The later bounces (b >= b0) of scenes with a light buffer in one
 // persistent launch: a lane carries a path of bounce b0's queue, whose next ray
 // hits, through all its remaining bounces in registers, and takes the next one
 // of its warp's share when it ends, so warps stay full while the queue lasts.
@@ -1515,7 +1517,7 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
             end(kFamExtend);
             ++nl;
             for (int b = 0; b < bounces; ++b) {
-                if (inl && b >= kPathsFrom) {   // the late bounces in one persistent launch
+                if (inl && b >= kPathsFrom<IS>) {   // the late bounces in one persistent launch
                     // on half the resident blocks: the late bounces are a trickle of
                     // paths, and the blocks stay resident until their pools drain,
                     // holding slots the other lanes' kernels could use (+1%)
@@ -1527,8 +1529,12 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
                 }
                 if (b > 0) {
                     begin(kFamExtend);
-                    if (inl) k_shade<G><<<shape.blocks_extend, kExtendThreads, 0, stream>>>(sc, ws, job, b);
-                    else k_bounce<IS><<<shape.blocks_extend, kExtendThreads, sm, stream>>>(sc, ws, job, b);
+                    if constexpr (IS == kIsBvh) {
+                        if (inl) k_shade<IS><<<shape.blocks_extend, kExtendThreads, 0, stream>>>(sc, ws, job, b);
+                        else k_bounce<IS><<<shape.blocks_extend, kExtendThreads, sm, stream>>>(sc, ws, job, b);
+                    } else {
+                        k_bounce<IS><<<shape.blocks_extend, kExtendThreads, sm, stream>>>(sc, ws, job, b);
+                    }
                     end(kFamExtend);
                     ++nl;
                 }
