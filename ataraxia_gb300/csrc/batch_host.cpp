@@ -308,11 +308,11 @@ atx_status Batch::autotune(uint32_t passes, atx_batch_tuning* chosen)
     for (auto& p : slots_)
         if (p && p->scene.view.use_bvh) any_bvh = true;
     // explicit values, so that putting the pick back restores them
-    if (!pick.bvh_leaf_size) pick.bvh_leaf_size = 16;
+    if (!pick.bvh_leaf_size) pick.bvh_leaf_size = 8;
     if (!pick.threads) pick.threads = 256;
     ATX_TRY(set_tuning(pick));
     if (any_bvh)
-        for (uint32_t leaf : {8u, 12u, 24u, 32u}) {
+        for (uint32_t leaf : {4u, 12u, 16u, 24u}) {
             atx_batch_tuning t = pick;
             t.bvh_leaf_size = leaf;
             ATX_TRY(trial(t));

@@ -18,7 +18,8 @@ namespace atx {
 namespace {
 constexpr uint32_t kDefaultWavePaths = 64u << 20;  // at most 64 Mi paths (8.7 GB of state) per wave
 constexpr uint32_t kDefaultBvhThreshold = 1025;  // LBVH above the direction buffer's 1,024 spheres (64-scene mix: +23% over 512)
-constexpr uint32_t kDefaultBvhLeaf = 16;   // fastest of 1..32 on the 65,536-sphere scene
+// of 16, 8 and 4: the 65,536-sphere scene 5.20, 4.96 and 4.95 ms a render, 8,000 spheres at 1280x720 2.63, 2.58 and 2.58 ms
+constexpr uint32_t kDefaultBvhLeaf = 8;
 constexpr uint32_t kMaxBounces = 4096;
 }  // namespace
 
@@ -1018,7 +1019,7 @@ atx_status Renderer::autotune(uint32_t spp, uint32_t passes, bool use_cache, atx
         return ATX_OK;
     };
     if (sv.use_bvh)
-        for (uint32_t leaf : {4u, 8u, 12u, 24u, 32u}) {
+        for (uint32_t leaf : {4u, 12u, 16u, 24u, 32u}) {
             atx_tuning t = best;
             t.bvh_leaf_size = leaf;
             ATX_TRY(trial(t));

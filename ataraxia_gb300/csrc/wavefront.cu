@@ -57,6 +57,22 @@ constexpr int kExtendBlocksPerSm = 4;
 template <int IS>
 constexpr int kPathsFrom = IS == kIsBvh ? 2 : 1;
 
+// LBVH scenes without cell lists: bounces from this one on run in one
+// persistent k_paths_walk launch.  It saves a walk launch and a shadow launch a
+// bounce, each as long as its longest ray, and loses k_bounce's full warps for
+// the shading, so the more paths a wave has the later it starts (us a render
+// with 6 spheres a leaf, from bounce 1 / 2 / 3 / 4 / never:
+//   50 K paths      74 /  101 /  106 /  111 /  148
+//   1.2 M          234 /  251 /  297 /  343 /  392
+//   2.1 M          587 /  529 /  552 /  602 /  738
+//   3.7 M         1815 / 1507 / 1437 / 1439
+//   7.4 M         3167 / 2616 / 2500 / 2474 / 2584
+//   4 x 8.3 M     5685 / 5194 / 4887 / 4778 / 4958).
+int walked_from(uint64_t paths)
+{
+    return paths <= (1u << 18) ? 1 : paths <= (1u << 21) ? 2 : paths <= (1u << 22) ? 3 : 4;
+}
+
 // k_shadow's blocks per SM: the shared-memory variant fits 40 registers
 // without spilling (6 blocks of 256 threads); the others take up to 64 (4).
 // k_fused's blocks per SM (whole paths in one thread: 64 registers).
@@ -132,7 +148,7 @@ __device__ __forceinline__ float4 light_dir(const SceneView& sc, uint32_t li, fl
 // step left 28 lanes idle, and a warp's walk a chain of every node it visits:
 // the lists of a 3840x2160 view of 65,536 spheres took 1,230 + 1,070 us, now
 // 370 + 270); a leaf cluster's spheres get the sphere test the brute-force masks
-// use, one per lane, two clusters of up to 16 at once.  All lanes call it with
+// use, one per lane, four clusters of up to 8 (or two of 16) at once.  All lanes call it with
 // the warp's own stack in shared memory.  Returns the number of candidates
 // (written to out when FILL), or kNoTileList when the walk overflows its stack
 // or step budget or the list would pass cap.
@@ -143,6 +159,7 @@ __device__ uint32_t tile_walk(const BvhView& b, const WarpCone& cone, float3 o, 
                               uint32_t cap)
 {
     const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
+    const uint32_t wide = b.leaf_size <= 8u ? 8u : b.leaf_size <= 16u ? 16u : 32u;   // lanes a leaf cluster gets
     uint32_t sp = 1u, count = 0u;
     uint32_t budget = 2u * b.n_leaves + 8u;
     __syncwarp();
@@ -177,17 +194,13 @@ __device__ uint32_t tile_walk(const BvhView& b, const WarpCone& cone, float3 o, 
         sp += (uint32_t)__popc(inner);
         __syncwarp();
         while (leaves) {
-            const int k = __ffs(leaves) - 1;
-            leaves &= leaves - 1u;
-            const int k2 = leaves ? __ffs(leaves) - 1 : k;
-            uint32_t first = __shfl_sync(kFull, ref, k), c = __shfl_sync(kFull, cnt, k);
-            const uint32_t first2 = __shfl_sync(kFull, ref, k2), c2 = __shfl_sync(kFull, cnt, k2);
-            uint32_t q = lane;
-            if (k2 != k && c <= 16u && c2 <= 16u) {   // lanes 16.. take the next cluster
-                leaves &= leaves - 1u;
-                if (lane >= 16u) first = first2, c = c2, q = lane - 16u;
-            }
-            c = min(c, b.n_leaves - first);
+            // lanes wide*i.. take the i-th of the next clusters
+            uint32_t mine = leaves;
+            for (uint32_t i = lane / wide; i; --i) mine &= mine - 1u;
+            const int from = mine ? __ffs(mine) - 1 : 0;
+            const uint32_t first = __shfl_sync(kFull, ref, from), held = __shfl_sync(kFull, cnt, from);
+            const uint32_t c = mine ? min(held, b.n_leaves - first) : 0u, q = lane % wide;
+            for (uint32_t i = 0; i < 32u / wide; ++i) leaves &= leaves - 1u;
             bool meets = false;
             if (q < c) {
                 const float4 s = __ldg(&b.leaf_sph[first + q]);
@@ -416,6 +429,22 @@ __device__ __forceinline__ Brdf load_mat(const SceneView& sc, int32_t mi)
     b.k = fabsf(m2.w);
     b.emits = __float_as_int(m2.w) < 0;
     return b;
+}
+
+// Whether the sphere a shadow ray leaves from (own, an index into the table)
+// occludes it, with the brute-force test.  Testing it first changes nothing
+// but the time: "occluded" means some sphere has t > 0 and t*t < dist2, in any
+// order (see occluded_brute).  A surface facing away from its light is
+// shadowed by its own sphere; the LBVH walk tests it first and skips the walk
+// (+5% on the 65,536-sphere scene).  The brute-force loop does not: there the
+// extra divergent test cost more than the chunks it saves (-2% on 256 spheres).
+__device__ __forceinline__ bool own_occludes(const SceneView& sc, const float4* sph, bool smem, uint32_t own,
+                                             float3 o, float3 d, float dist2)
+{
+    if (own >= sc.n_sph) return false;
+    const float4 s = smem ? smem_sphere(sph, own) : __ldg(&sc.sph[own]);
+    float t;
+    return sphere_t(s, o, d, dot3(d, d), t) && t > 0.0f && t * t < dist2;
 }
 
 // What shading a hit leaves behind (Renderer.cu:318-384 for one bounce).
@@ -887,20 +916,86 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
     warp_push_n(&ws.counters[2 * b0 + 1], traced);
 }
 
-// Whether the sphere a shadow ray leaves from (own, an index into the table)
-// occludes it, with the brute-force test.  Testing it first changes nothing
-// but the time: "occluded" means some sphere has t > 0 and t*t < dist2, in any
-// order (see occluded_brute).  A surface facing away from its light is
-// shadowed by its own sphere; the LBVH walk tests it first and skips the walk
-// (+5% on the 65,536-sphere scene).  The brute-force loop does not: there the
-// extra divergent test cost more than the chunks it saves (-2% on 256 spheres).
-__device__ __forceinline__ bool own_occludes(const SceneView& sc, const float4* sph, bool smem, uint32_t own,
-                                             float3 o, float3 d, float dist2)
+// The late bounces (b >= b0) of LBVH scenes without cell lists in one launch, as
+// k_paths, with both rays of a bounce walked where they are: the queue's rays
+// are not traced yet, so a round traces, shades, tests the shadow ray and turns.
+// These bounces hold few rays, and a launch each for their walks and their
+// shadow rays was mostly waiting: for the longest walk of each, and for
+// nothing at all (walked_from has the times).
+__global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
+    k_paths_walk(SceneView sc, WaveState ws, WaveJob job, int b0)
 {
-    if (own >= sc.n_sph) return false;
-    const float4 s = smem ? smem_sphere(sph, own) : __ldg(&sc.sph[own]);
-    float t;
-    return sphere_t(s, o, d, dot3(d, d), t) && t > 0.0f && t * t < dist2;
+    const uint32_t n0 = ws.counters[2 * b0];   // bounce b0's queue
+    const uint32_t lane = lane_id();
+    // the warp's share: chunks of 32 entries, one in every grid's worth of warps
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    uint32_t chunk = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u, used = 0u;   // warp-uniform
+    if (chunk * 32u >= n0) return;
+    const uint32_t* q0 = (b0 & 1) ? ws.q[1] : ws.q[0];
+    uint32_t rays = 0u, traced = 0u;   // continuation rays made here, shadow rays
+    bool live = false;
+    uint32_t pid = 0u, b = 0u, seed = 0u;
+    float3 o = mk3(0.f, 0.f, 0.f), d = o, thr = o;
+
+    for (;;) {   // ends: every round takes each live path a bounce further or off
+        uint32_t idle = __ballot_sync(kFull, !live);
+        while (idle && chunk * 32u < n0) {   // lanes without a path take the next of the share
+            const uint32_t have = min(32u, n0 - chunk * 32u) - used;
+            const uint32_t rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (!live && rank < have) {
+                pid = q0[chunk * 32u + used + rank];
+                const float4 ro = ws.ray_o[pid];
+                const float4 rd = ws.ray_d[pid];
+                const float4 tt = ws.thr[pid];
+                o = mk3(ro.x, ro.y, ro.z);
+                seed = __float_as_uint(ro.w);
+                d = mk3(rd.x, rd.y, rd.z);
+                thr = mk3(tt.x, tt.y, tt.z);
+                b = (uint32_t)b0;
+                live = true;
+            }
+            used += min((uint32_t)__popc(idle), have);
+            if (used == min(32u, n0 - chunk * 32u)) {
+                chunk += warps;
+                used = 0u;
+            }
+            idle = __ballot_sync(kFull, !live);
+        }
+        if (idle == kFull) break;
+        if (live) {
+            float tmin;
+            const int32_t hit = bvh_nearest(sc.bvh, o, d, tmin);
+            Shaded r{};
+            bool sky = false;
+            if (hit >= 0) {
+                uint32_t own = ~0u;
+                seed += b;
+                const bool last = (int)b + 1 >= job.max_bounces;
+                shade_hit<kIsBvh, false>(sc, sc.sph, ws, pid, hit, tmin, o, d, thr, own, seed, last, r);
+                if (r.push_sh) {
+                    ++traced;
+                    const float3 so = mk3(r.sho.x, r.sho.y, r.sho.z), sd = mk3(r.shd.x, r.shd.y, r.shd.z);
+                    r.lit = !own_occludes(sc, sc.sph, false, (uint32_t)hit, so, sd, r.sho.w) &&
+                            !bvh_occluded(sc.bvh, so, sd, r.sho.w);
+                    r.lc = mk3(r.shc.x, r.shc.y, r.shc.z);
+                }
+                rays += r.push_next ? 1u : 0u;
+            } else {
+                sky = job.sky != 0;   // Renderer.cu:311-316: the path ends in the sky
+            }
+            if (r.touch || r.lit || sky) {
+                const float4 c0 = ws.col[pid];
+                float3 c = bounce_terms(mk3(c0.x, c0.y, c0.z), r);
+                if (sky) c = sky_term(c, thr);
+                ws.col[pid] = make_float4(c.x, c.y, c.z, c0.w);
+            }
+            live = r.push_next;
+            ++b;
+        }
+    }
+    // statistics, as k_paths keeps them (bounce b0's queue is counted already)
+    warp_push_n(&ws.counters[2 * ((uint32_t)job.max_bounces + 1u) + 3u], rays);
+    warp_push_n(&ws.counters[2 * b0 + 1], traced);
 }
 
 // A shadow ray of one bounce's queue: origin, direction, squared distance to
@@ -1523,6 +1618,13 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
                     // holding slots the other lanes' kernels could use (+1%)
                     begin(kFamExtend);
                     k_paths<G><<<max(1, shape.blocks_extend / 2), kExtendThreads, 0, stream>>>(sc, ws, job, b);
+                    end(kFamExtend);
+                    ++nl;
+                    break;
+                }
+                if (IS == kIsBvh && !inl && b >= walked_from(paths)) {
+                    begin(kFamExtend);
+                    k_paths_walk<<<max(1, shape.blocks_extend / 2), kExtendThreads, 0, stream>>>(sc, ws, job, b);
                     end(kFamExtend);
                     ++nl;
                     break;

@@ -100,7 +100,7 @@ typedef struct atx_config {
     uint32_t wave_paths;       /* paths in flight per wave; 0 = autotuned default */
     uint32_t threads;          /* threads per block; 0 = default */
     uint32_t bvh_threshold;    /* sphere count at which the LBVH replaces the brute-force tables; 0 = 1025 */
-    uint32_t bvh_leaf_size;    /* spheres per BVH leaf; 0 = 16, or what atx_autotune picks */
+    uint32_t bvh_leaf_size;    /* spheres per BVH leaf; 0 = 8, or what atx_autotune picks */
     uint32_t flags;            /* ATX_FLAG_* */
     uint64_t hbm_budget_bytes; /* device bytes this renderer may hold; 0 = unlimited */
 } atx_config;
@@ -240,7 +240,7 @@ ATX_API atx_status atx_get_stream(atx_renderer* r, void** stream);
  * Every setting renders the same frames bit for bit; only speed changes.  A
  * zero field means the default. */
 typedef struct atx_tuning {
-    uint32_t bvh_leaf_size;    /* spheres per LBVH leaf cluster (LBVH scenes; default 16) */
+    uint32_t bvh_leaf_size;    /* spheres per LBVH leaf cluster (LBVH scenes; default 8) */
     uint32_t lanes;            /* concurrent lanes (streams with their own path state) a launch is split over */
     uint32_t wave_paths;       /* path state per lane, paths (default: sized to the launch, up to 64 Mi) */
     uint32_t threads;          /* threads per block of the primary and shadow kernels (multiple of 32, <= 256) */
