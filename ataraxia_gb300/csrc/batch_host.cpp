@@ -413,8 +413,8 @@ atx_status Batch::run(cudaEvent_t done)
     for (uint32_t l = 0; l < nl; ++l)
         for (uint32_t k : plan[l]) now_lanes[parts[k].id] |= 1ull << l;
 
-    // The graph's shape: lanes, their parts in order, whether each clears its
-    // accumulator rows, its waves and bounces.  A pass of the same shape as
+    // The graph's shape: lanes, their parts in order, whether each starts its
+    // accumulator rows from zero, its waves and bounces.  A pass of the same shape as
     // the last one replays the graph with updated kernel arguments; a pass of
     // a new shape (scenes come and go in a server) is launched directly,
     // since capturing and instantiating a graph used once costs more host time.
@@ -468,11 +468,6 @@ atx_status Batch::run(cudaEvent_t done)
             for (uint32_t k : plan[l]) {
                 const Part& q = parts[k];
                 Slot* s = slots_[q.id].get();
-                if (frame0[q.id] == 1) {
-                    ATX_CUDA(enqueue_clear_accum(s->accum.as<float4>() + q.pix_begin, q.pix_end - q.pix_begin,
-                                                 ln.stream));
-                    ++launches;
-                }
                 waves += (uint32_t)part_waves(q, ln.wave.view.capacity);
                 ATX_TRY(enqueue_frames(s->scene.view, s->cam, ln.wave, s->shape, frame0[q.id], s->spp_next,
                                        s->settings.max_bounces, s->settings.sky_light ? 1 : 0, s->accum.as<float4>(),

@@ -170,11 +170,10 @@ extern "C" ATX_API atx_status atx_render_noalloc(const atx_sphere* spheres, uint
     LaunchShape shape{};
     ATX_CUDA(plan_launch(sc, device, 0, &shape));
 
-    // Renderer.cu:181-182 / :245-248: frame 1 starts from a cleared
-    // accumulator; with accumulation off the frames are 1..spp
+    // Renderer.cu:181-182 / :245-248: frame 1 starts the accumulator from zero;
+    // with accumulation off the frames are 1..spp
     const uint32_t f0 = settings->accumulation ? frame_index : 1u;
     float4* acc = reinterpret_cast<float4*>(accumulation);
-    if (f0 == 1) ATX_CUDA(enqueue_clear_accum(acc, (uint64_t)width * height, st));
 
     const uint64_t pixels = (uint64_t)width * height;
     const WavePlan plan = plan_waves(pixels, spp, capacity);
@@ -193,6 +192,7 @@ extern "C" ATX_API atx_status atx_render_noalloc(const atx_sphere* spheres, uint
             job.pack_frame = (s0 + job.spp >= spp && image) ? last_frame : 0u;
             job.prim_cache = nullptr;
             job.prim_cached = 0;
+            job.fresh = f0 == 1u && s0 == 0u ? 1 : 0;
             ATX_CUDA(enqueue_wave(sc, cam, ws, job, shape, acc, image, st, &launches, nullptr));
         }
     }

@@ -209,10 +209,13 @@ private:
     uint64_t tickets_ = 0;
     uint32_t* image_buf(int i) { return (i ? image_alt_ : image_).as<uint32_t>(); }
     // Primary directions for the camera they were computed for (dirs_cam_):
-    // rebuilt when the camera's matrices or the viewport change.
+    // rebuilt for new matrices or a new viewport once two renders had them.
     DeviceBuffer dirs_;
     CameraView dirs_cam_{};
     bool dirs_valid_ = false;
+    CameraView last_dirs_{};         // the previous render's camera
+    bool last_dirs_valid_ = false;
+    bool dirs_due() const;
     // Primary tile masks for the camera, eye and scene they were built for
     // (masks_cam_; scenes on the brute-force tables up to 1,024 spheres):
     // rebuilt when any of them changes.

@@ -1160,7 +1160,7 @@ __global__ void __launch_bounds__(kThreads) k_accumulate(WaveState ws, WaveJob j
     const float fspp = __uint2float_rn(job.spp);
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < job.n_pixels; j += stride) {
         const uint32_t p = job.pixel0 + j;
-        float4 a = accum[p];
+        float4 a = job.fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : accum[p];
         const bool missed = job.max_bounces > 0 && (int32_t)prim[j].y < 0;
         // Every sample adds (0, 0, 0) and a frame (a missed primary without
         // sky light, or no bounces): the spp additions of 0 leave x, y, z as
@@ -1235,7 +1235,7 @@ __global__ void __launch_bounds__(kThreads, kFusedBlocksPerSm) k_fused(SceneView
                 if (job.prim_cache) job.prim_cache[p] = make_uint2(__float_as_uint(t0), (uint32_t)h0);
             }
         }
-        float4 a = accum[p];
+        float4 a = job.fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : accum[p];
         uint32_t known = 0u, seen = 0u;   // bounce-0 lights tested from this pixel's hit, and the visible ones
         for (uint32_t s = 0; s < job.spp; ++s) {
             float3 c = mk3(0.f, 0.f, 0.f);
@@ -1314,13 +1314,6 @@ __global__ void __launch_bounds__(kThreads, kFusedBlocksPerSm) k_fused(SceneView
             if (n_first) atomicAdd(&ws.totals[2], (unsigned long long)n_first);
         }
     }
-}
-
-__global__ void k_clear(float4* p, uint64_t n)
-{
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 template <int IS>
@@ -1653,12 +1646,6 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
     end(kFamAccumulate);
     ++nl;
     if (launches) *launches += nl;
-    return cudaGetLastError();
-}
-
-cudaError_t enqueue_clear_accum(float4* accum, uint64_t n, cudaStream_t stream)
-{
-    k_clear<<<grid_for(n, kThreads, 4096), kThreads, 0, stream>>>(accum, n);
     return cudaGetLastError();
 }
 

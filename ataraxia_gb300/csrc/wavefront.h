@@ -278,6 +278,10 @@ struct WaveJob {
     // holds this view's hits, so they are not traced again.
     uint2* prim_cache;
     int32_t prim_cached;
+    // The wave's samples are the first of these pixels (frame 1): the
+    // accumulator starts from zero instead of being read (Renderer.cu:181-182
+    // clears it).
+    int32_t fresh;
     uint64_t spp_div;         // fastmod_multiplier(spp), set by enqueue_wave: x / spp by multiplication
 };
 
@@ -335,9 +339,6 @@ cudaError_t plan_launch(const SceneView& sc, int device, int threads, LaunchShap
 cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveState& ws, const WaveJob& job,
                          const LaunchShape& shape, float4* accum, uint32_t* image, cudaStream_t stream,
                          uint32_t* launches, KernelTimer* timer = nullptr);
-
-// Zeroes n float4 on stream.
-cudaError_t enqueue_clear_accum(float4* accum, uint64_t n, cudaStream_t stream);
 
 // Debug / parity hook: nearest hit for n rays through the same device code the
 // renderer uses.  origins/dirs are 3 floats per ray in device memory.
