@@ -1545,7 +1545,8 @@ cudaError_t plan_launch(const SceneView& sc, int device, int threads, LaunchShap
     out->blocks_primary = sms * (pr > 0 ? pr : 1);
     out->smem_spheres = bytes;
     out->mode = mode;
-    out->fused = mode == kIsBvh ? 0 : path_kernel == 2 ? 2 : (path_kernel == 0 && sc.n_sph <= kFusedMaxSpheres) ? 1 : 0;
+    out->fused = mode == kIsBvh ? 0 : path_kernel == 2 ? 2 : path_kernel != 0 ? 0 :
+                 sc.n_sph <= kFusedMaxSpheres ? 1 : sc.n_sph <= kFusedSmallSpheres ? 3 : 0;
     return cudaSuccess;
 }
 
@@ -1561,7 +1562,9 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
     const uint64_t paths = (uint64_t)job.n_pixels * job.spp;
     auto begin = [&](int fam) { if (timer) timer->begin(fam, stream); };
     auto end = [&](int fam) { if (timer) timer->end(fam, stream); };
-    if (shape.mode != kIsBvh && (shape.fused == 2 || (shape.fused == 1 && job.spp <= kFusedMaxSpp))) {
+    const bool small = job.spp <= kFusedMaxSpp && paths * job.spp * sc.n_sph <= kFusedSmallWork;
+    if (shape.mode != kIsBvh && (shape.fused == 2 || (shape.fused == 1 && job.spp <= kFusedMaxSpp) ||
+                                 (shape.fused == 3 && small))) {
         // whole paths in one thread per pixel
         const int g = grid_for(job.n_pixels, kThreads, 1 << 20);
         begin(kFamExtend);

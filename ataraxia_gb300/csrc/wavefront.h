@@ -316,17 +316,26 @@ struct LaunchShape {
     int threads;
     size_t smem_spheres;      // dynamic shared memory for the sphere table (0: read from global)
     int mode;                 // nearest-hit structure: 0 brute force from global, 1 from shared memory, 2 LBVH
-    int fused;                // whole paths in one thread (k_fused): 0 never, 1 for waves of at most
-                              // kFusedMaxSpp samples per pixel, 2 always (brute-force tables only)
+    int fused;                // whole paths in one thread (k_fused, brute-force tables only): 0 never, 1 for
+                              // waves of at most kFusedMaxSpp samples per pixel, 2 always, 3 for small waves
+                              // (kFusedSmallWork)
 };
 
-// Scenes of at most this many spheres on the brute-force tables render waves
-// of at most kFusedMaxSpp samples per pixel with whole paths in one thread
-// unless told otherwise (small scene: 1 sample per call +38%, 8 about even,
-// 64 -16% against the wavefront stages, whose shared first-bounce work pays
-// with many samples).
+// Scenes of at most kFusedMaxSpheres spheres on the brute-force tables render
+// waves of at most kFusedMaxSpp samples per pixel with whole paths in one thread
+// unless told otherwise (9 spheres at 1280x720: 1 sample per call 77 against 100
+// us with the wavefront stages, 4 even, 8 436 against 410, whose shared
+// first-bounce work pays with many samples).  So do scenes of up to
+// kFusedSmallSpheres in waves so small that the stages' launches and the chain
+// through them are most of it: spheres x pixels x samples^2 up to
+// kFusedSmallWork (30 spheres, 640x480, 1 sample: 12.7 against 21.2 us, 2 samples
+// 17.7 against 25.0; 64 spheres, 256x256: 11.2 against 19.6, 640x480: 19.9 against
+// 23.1; past it, 64 spheres at 1280x720 45 against 32, 4 samples at 256x256 26
+// against 23).
 constexpr uint32_t kFusedMaxSpheres = 24;
 constexpr uint32_t kFusedMaxSpp = 8;
+constexpr uint32_t kFusedSmallSpheres = 64;
+constexpr uint64_t kFusedSmallWork = 40000000;
 
 // Fills in grid sizes for this device and scene (occupancy-derived).
 // path_kernel: 0 by scene size, 1 the wavefront stages, 2 whole paths in one
