@@ -216,6 +216,9 @@ __device__ __forceinline__ float3 sample_next(const Brdf& m, float3 t, float3 b,
 // truncating x*255 per channel, packed A<<24 | B<<16 | G<<8 | R.
 __device__ __forceinline__ uint32_t pack_rgba8(float4 acc, float frame)
 {
+    // a background pixel: 0 / frame is 0 and frame / frame is 1 (most of an open
+    // scene's image, without its four IEEE divisions)
+    if (acc.x == 0.0f && acc.y == 0.0f && acc.z == 0.0f && acc.w == frame && frame > 0.0f) return 0xff000000u;
     float v[4] = { acc.x / frame, acc.y / frame, acc.z / frame, acc.w / frame };
     uint32_t ch[4];
 #pragma unroll

@@ -506,8 +506,8 @@ __device__ __forceinline__ bool all_occluded(const SceneView& sc, const float4* 
 
 // Cell of direction w around a light, as light_buffer.cu lays out the cube:
 // the face of the largest |component| (+x, -x, +y, -y, +z, -z), then the other
-// two components over it (in [-1, 1]) on a res x res grid.  -1 for a zero or
-// non-finite w.
+// two components over it (in [-1, 1]) on a res x res grid.  -1 for a w that is
+// not finite, or so long or short that the quotient below may not be good.
 __device__ __forceinline__ int lb_cell(float3 w, uint32_t res)
 {
     const float ax = fabsf(w.x), ay = fabsf(w.y), az = fabsf(w.z);
@@ -523,8 +523,9 @@ __device__ __forceinline__ int lb_cell(float3 w, uint32_t res)
         face = w.z >= 0.0f ? 4u : 5u;
         m = az, a = w.x, b = w.y;
     }
-    if (!(m > 0.0f && m < 3.0e38f) || !(fabsf(a) <= m && fabsf(b) <= m)) return -1;
-    const float h = 0.5f * (float)res / m;
+    if (!(m > 1.0e-30f && m < 8.0e37f) || !(fabsf(a) <= m && fabsf(b) <= m)) return -1;
+    // within 2 ulp for these m; the cells' cones are widened by 2e-4 rad
+    const float h = __fdividef(0.5f * (float)res, m);
     const int i = min((int)((a + m) * h), (int)res - 1);
     const int j = min((int)((b + m) * h), (int)res - 1);
     return (int)((face * res + (uint32_t)i) * res + (uint32_t)j);
