@@ -640,14 +640,16 @@ atx_status Renderer::render(uint32_t spp)
     // to the lane count for the scene (at least 4 Mi paths each), one lane
     // when the caller fixed the wave size or kernels are being timed one by
     // one.  Scenes with light and direction buffers run their late bounces in
-    // one persistent launch and, with each render joined, overlap best on two
-    // lanes; LBVH scenes, and every scene with overlapped renders (whose lanes
-    // run on from one render into the next), use four (large scene: 4 lanes
-    // +11% over 2; medium scene overlapped: 4 lanes +12% over 2).
+    // one persistent launch and overlap best on two lanes with each render
+    // joined, on three with overlapped renders, whose lanes run on from one
+    // render into the next (medium scene: one renderer 254 us a render, 257 with
+    // four; three in turn 238 against 252).  LBVH scenes use four (65,536 spheres,
+    // one renderer: 5.20, 5.04 and 5.12 ms on two, three and four; 4,096 with cell
+    // lists: 903, 867 and 840 us).
     const uint64_t px = (uint64_t)width_ * height_;
     const bool profile = (cfg_.flags & ATX_FLAG_PROFILE_KERNELS) != 0;
-    uint32_t max_lanes = (!overlap_ && !scene_.view.use_bvh && scene_.view.lb.n_lights) ? kBufferedLanes
-                                                                                         : kDefaultLanes;
+    uint32_t max_lanes = kDefaultLanes;
+    if (!scene_.view.use_bvh && scene_.view.lb.n_lights) max_lanes = overlap_ ? kOverlappedLanes : kBufferedLanes;
     if (tune_.lanes) max_lanes = std::min<uint32_t>(tune_.lanes, kLanes);
     const uint32_t wave_paths = tune_.wave_paths ? tune_.wave_paths : cfg_.wave_paths;
     // at least 4 Mi paths per lane

@@ -175,8 +175,9 @@ private:
     // bounces overlap the others' work instead of leaving SMs idle.  Lane 0
     // is the renderer's stream.
     static constexpr int kLanes = 8;
-    static constexpr int kDefaultLanes = 4;    // LBVH scenes, and any scene with overlapped renders
-    static constexpr int kBufferedLanes = 2;   // scenes with light and direction buffers, renders joined
+    static constexpr int kDefaultLanes = 4;      // LBVH scenes, scenes without a light buffer
+    static constexpr int kBufferedLanes = 2;     // scenes with light and direction buffers, renders joined
+    static constexpr int kOverlappedLanes = 3;   // and with overlapped renders
     WaveStore wave_[kLanes];
     cudaStream_t lane_stream_[kLanes] = {};
     cudaEvent_t fork_ = nullptr, join_[kLanes] = {};
