@@ -545,6 +545,7 @@ atx_status Batch::read_accumulation(uint32_t id, float* host, uint64_t n)
     if (!s) return fail(ATX_ERR_NOT_FOUND, "batch: no scene %u", id);
     if (!host || n > (uint64_t)s->w * s->h) return fail(ATX_ERR_INVALID_ARG, "batch_read_accumulation: bad buffer");
     ATX_CUDA(cudaSetDevice(cfg_.device));
+    prefault(host, n * sizeof(float4));   // while the passes run
     ATX_CUDA(cudaMemcpyAsync(host, s->accum.get(), n * sizeof(float4), cudaMemcpyDeviceToHost, stream_));
     ATX_CUDA(cudaStreamSynchronize(stream_));
     return ATX_OK;
@@ -556,6 +557,7 @@ atx_status Batch::read_image(uint32_t id, uint32_t* host, uint64_t n)
     if (!s) return fail(ATX_ERR_NOT_FOUND, "batch: no scene %u", id);
     if (!host || n > (uint64_t)s->w * s->h) return fail(ATX_ERR_INVALID_ARG, "batch_read_image: bad buffer");
     ATX_CUDA(cudaSetDevice(cfg_.device));
+    prefault(host, n * sizeof(uint32_t));   // while the passes run
     ATX_CUDA(cudaMemcpyAsync(host, s->image.get(), n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_));
     ATX_CUDA(cudaStreamSynchronize(stream_));
     return ATX_OK;

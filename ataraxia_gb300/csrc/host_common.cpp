@@ -3,6 +3,11 @@
 // and aarch64.
 #include "host_common.h"
 
+#if defined(__linux__)
+#include <sys/mman.h>
+#include <unistd.h>
+#endif
+
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -55,6 +60,22 @@ atx_status DeviceBuffer::ensure(uint64_t bytes, Budget* budget, const char* what
     bytes_ = bytes;
     budget_ = budget;
     return ATX_OK;
+}
+
+void prefault(void* p, uint64_t bytes)
+{
+#if defined(__linux__)
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+    static const uint64_t page = (uint64_t)sysconf(_SC_PAGESIZE);
+    if (bytes < (256u << 10)) return;
+    const uint64_t a = ((uint64_t)(uintptr_t)p + page - 1) / page * page, b = ((uint64_t)(uintptr_t)p + bytes) / page * page;
+    if (b > a) (void)madvise(reinterpret_cast<void*>((uintptr_t)a), b - a, MADV_POPULATE_WRITE);
+#else
+    (void)p;
+    (void)bytes;
+#endif
 }
 
 void DeviceBuffer::reset()

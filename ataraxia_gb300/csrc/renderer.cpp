@@ -761,6 +761,7 @@ atx_status Renderer::read_accumulation(float* host, uint64_t n)
                                                     (unsigned long long)n);
     ATX_TRY(activate());
     ATX_TRY(join());
+    prefault(host, n * sizeof(float4));   // while the renders run
     ATX_CUDA(cudaMemcpyAsync(host, accum_.get(), n * sizeof(float4), cudaMemcpyDeviceToHost, stream_));
     ATX_CUDA(cudaStreamSynchronize(stream_));
     return ATX_OK;
@@ -773,6 +774,7 @@ atx_status Renderer::read_image(uint32_t* host, uint64_t n)
                                                     (unsigned long long)n);
     ATX_TRY(activate());
     ATX_TRY(join());
+    prefault(host, n * sizeof(uint32_t));   // while the renders run
     ATX_CUDA(cudaMemcpyAsync(host, image_buf(img_last_), n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_));
     ATX_CUDA(cudaStreamSynchronize(stream_));
     return ATX_OK;
