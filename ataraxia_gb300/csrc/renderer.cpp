@@ -129,9 +129,9 @@ bool SceneStore::lists_due(uint64_t paths)
     const uint64_t n = view.n_sph;
     if (!view.use_bvh || lists_tried || n > kDbMaxBvhSpheres || view.n_lights == 0 || view.n_lights > kLbMaxLights)
         return false;
-    // The build takes 5.8 ms at 4,096 spheres and goes with their square; a path
-    // over the lists instead of the tree saves 0.17 ns there (16 samples of
-    // 1280x720 pixels: 3.28 against 0.76 ms), so it pays after about 2 n^2 paths.
+    // The build takes 7.5 ms at 4,096 spheres, 39 at 8,000, and a path over the
+    // lists instead of the tree saves 0.17 and 0.24 ns there (16 samples of
+    // 1280x720 pixels), so it pays after about 2 n^2 paths.
     // The call at hand counts for an eighth of its paths: a scene uploaded for
     // every render would build its lists each time (1,471 clustered spheres, 4
     // samples of 2560x1440 pixels: 1.13 against 0.79 ms).
@@ -147,7 +147,7 @@ void SceneStore::build_lists(Budget* budget, cudaStream_t stream)
     const uint64_t lb = lb_bytes(nl, kBvhLightRes, kBvhLine), db = db_bytes(n, kBvhDirRes, kBvhLine);
     if (budget && budget->cap()) return;   // what fitted the caller's budget still has to
     size_t free = 0, total = 0;
-    if (cudaMemGetInfo(&free, &total) != cudaSuccess || (lbuf.bytes() + dbuf.bytes() < lb + db && (lb + db) > free / 4)) {
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess || (lbuf.bytes() + dbuf.bytes() < lb + db && (lb + db) > free / 16)) {
         (void)cudaGetLastError();
         return;
     }

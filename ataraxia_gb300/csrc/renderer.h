@@ -43,7 +43,7 @@ struct SceneStore {
     // have paid for the build; a scene rendered once, or uploaded for every render, keeps
     // to the tree.  build_lists leaves the scene on the tree when a budget is
     // set, which later buffers may need in full, or when the lists would take
-    // more than a quarter of the device's free memory.
+    // more than a sixteenth of the device's free memory.
     bool lists_due(uint64_t paths);
     void build_lists(Budget* budget, cudaStream_t stream);
     uint64_t paths_seen = 0;    // since the upload, until the lists were tried

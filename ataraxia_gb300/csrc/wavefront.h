@@ -128,12 +128,13 @@ constexpr uint32_t kDbMaxSpheres = 1024;   // 393 KB of cells per sphere at res 
 // traced enough paths to pay for the build (SceneStore::lists_due), at these
 // resolutions and with lines twice as long (63 spheres).  A lookup and a few
 // spheres replace a walk that runs 5 to 9 of a warp's 32 lanes: 16 samples of
-// 1280x720 pixels over 4,096 spheres 3.28 -> 0.76 ms.  The walk is left for
-// cells whose list overflowed, 0.2% of the extension rays there; with 64-byte
-// lines at 32 cells 1% (1.23 ms), at 16 cells 10%.  Beyond, lists and build
-// grow (442 KB a sphere, every pair looked at) and clusters overflow them.
-constexpr uint32_t kDbMaxBvhSpheres = 4096;
-constexpr uint32_t kBvhDirRes = 24;
+// 1280x720 pixels over 4,096 spheres 3.05 -> 0.56 ms (0.66 at 24 cells, 1.23 with
+// 64-byte lines, whose lists overflow for 1% of the extension rays), over 8,000
+// 4.82 -> 1.32 (2.08 at 24), 8,000 in clusters 0.33 -> 0.22.  The walk is left for
+// cells whose list overflowed.  Beyond, lists and build grow (786 KB a sphere,
+// every pair looked at) and more of them overflow.
+constexpr uint32_t kDbMaxBvhSpheres = 8192;
+constexpr uint32_t kBvhDirRes = 32;
 constexpr uint32_t kBvhLightRes = 64;   // a light sees the whole scene behind a cell: finer cells than a sphere's
 constexpr uint32_t kBvhLine = 64;       // 16-bit words per cell
 struct DirBufferView {

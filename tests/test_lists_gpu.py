@@ -46,7 +46,8 @@ def _render(sc, calls, sky, **kw):
 # the smallest LBVH scene, one in between and the most spheres with lists; the calls' paths pass
 # 2 n^2 with the second call
 @pytest.mark.parametrize("kind,n,lights,sky", [("open", 1025, 1, False), ("clump", 1300, 5, True),
-                                               ("tied", 1401, 40, False), ("open", 4096, 8, False)])
+                                               ("tied", 1401, 40, False), ("open", 4096, 8, False),
+                                               ("clump", 8192, 3, False)])
 @pytest.mark.parametrize("flags", [0, _native.FLAG_OVERLAP_RENDERS])
 def test_lists_render_as_the_general_path(kind, n, lights, sky, flags):
     sc = _scene(kind, n, lights)
