@@ -396,23 +396,19 @@ __global__ void __launch_bounds__(kThreads, IS == kIsBvh ? 4 : 5) k_primary(Scen
             r.p = p;
             store_record(ws, slot, r);
         }
-        // one slot range per warp, lane after lane: an inclusive scan of the
-        // lanes' light counts and one atomicAdd
-        const uint32_t cnt = (uint32_t)__popc(lights);
-        uint32_t incl = cnt;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFull, incl, off);
-            if ((int)lane_id() >= off) incl += v;
-        }
-        const uint32_t total = __shfl_sync(kFull, incl, 31);
-        uint32_t at = 0u;
-        if (lane_id() == 31u && total) at = atomicAdd(&ws.counters[1], total);
-        at = __shfl_sync(kFull, at, 31) + incl - cnt;
-        while (lights) {
-            const uint32_t li = (uint32_t)(__ffs(lights) - 1);
-            lights &= lights - 1u;
-            ws.q[0][at++] = shadow_tag(slot, li);
+        // one slot range per warp, light after light: neighbouring entries are rays
+        // of neighbouring pixels towards one light
+        const uint32_t total = __reduce_add_sync(kFull, (uint32_t)__popc(lights));
+        uint32_t rest = __reduce_or_sync(kFull, lights), at = 0u;
+        if (lane_id() == 0u && total) at = atomicAdd(&ws.counters[1], total);
+        at = __shfl_sync(kFull, at, 0);
+        while (rest) {
+            const uint32_t li = (uint32_t)(__ffs(rest) - 1);
+            rest &= rest - 1u;
+            const bool mine = ((lights >> li) & 1u) != 0u;
+            const uint32_t m = __ballot_sync(kFull, mine);
+            if (mine) ws.q[0][at + (uint32_t)__popc(m & ((1u << lane_id()) - 1u))] = shadow_tag(slot, li);
+            at += (uint32_t)__popc(m);
         }
     }
 }
