@@ -176,12 +176,13 @@ __device__ __forceinline__ void bvh_order(float& ta, uint32_t& ra, uint32_t& ca,
     }
 }
 
-// Stack depth.  Each step pops one node and pushes at most four, all one
-// 4-wide level down, so the stack holds at most three entries per level plus
-// one.  A Karras tree over 30-bit codes made distinct by the sorted position
-// is at most 30 + ceil(log2 n) binary levels deep, 62 for n = 2^32, so at most
-// 31 4-wide levels: 94 entries.
-constexpr int kBvhStack = 96;
+// Stack depth.  Each step pops one node and pushes at most four of its
+// descendants, so below every node on the way to the one at hand at most three
+// entries wait, plus one.  A step goes down at least one binary level (two on
+// average; a child is left closed when the other one's descendants are larger),
+// and a Karras tree over 30-bit codes made distinct by the sorted position is
+// at most 30 + ceil(log2 n) levels deep, 62 for n = 2^32: 187 entries.
+constexpr int kBvhStack = 192;
 
 __device__ __forceinline__ int32_t bvh_nearest(const BvhView& b, float3 o, float3 d, float& tmin)
 {

@@ -12,7 +12,7 @@
 //      over (code, sorted position), which makes every key distinct
 //   5. bottom-up boxes: each leaf thread climbs, the second arrival at a node
 //      forms the union of its children's boxes
-//   6. 4-wide nodes for traversal (the four grandchildren's boxes in two
+//   6. 4-wide nodes for traversal (the boxes of four descendants in two
 //      lines, subtrees of at most leaf_size spheres collapsed into leaf
 //      clusters)
 #include <cstdint>
@@ -281,33 +281,54 @@ __device__ PackedChild pack_child(int n, uint32_t leaf_size, const float4* node_
     return r;
 }
 
-// 4-wide nodes for traversal: internal node i stores the boxes of its four
-// grandchildren (a child that is a leaf cluster stands in for its own two
-// slots, with an empty second slot: ref = ~0, cnt = 0), so one traversal step
-// descends two levels of the binary tree.  Eight float4 rows (two 64-byte
-// lines); rows 4j..4j+3 hold slots 2j and 2j+1 interleaved component by
-// component, so one packed f32x2 instruction does a step of two box tests:
+// 4-wide nodes for traversal: internal node i stores the boxes of four of its
+// descendants that together hold its spheres: its two children, of which the
+// internal one with the largest surface is replaced by its own two children
+// until there are four (fewer when only leaf clusters are left: an empty slot
+// has ref = ~0, cnt = 0).  Always taking the four grandchildren left a slot
+// empty beside every leaf cluster and opened small boxes before large ones.
+// Against it, renders of clustered scenes: 65,536 spheres at 3840x2160, 4
+// samples, 4.74 -> 4.53 ms; 20,000 1.68 -> 1.57; 8,193 at 853x479, 1 sample, 116
+// -> 109 us; spheres spread evenly +-0.3%, whose trees are even too.
+// Eight float4 rows (two 64-byte lines); rows 4j..4j+3 hold slots 2j and 2j+1
+// interleaved component by component, so one packed f32x2 instruction does a
+// step of two box tests:
 // (cx_a, cx_b, cy_a, cy_b), (cz_a, cz_b, hx_a, hx_b), (hy_a, hy_b, hz_a, hz_b),
 // (ref_a, ref_b, cnt_a, cnt_b), with c the box centre and h its half extent.
 // An internal slot's ref is a binary node index, whose own 4-wide node holds
-// its grandchildren; nodes at odd depths are built but never visited.
+// its descendants; nodes that were opened are built but never visited.
 __global__ void k_pack_quads(int n, uint32_t leaf_size, const float4* node_ctr, const float4* node_half,
                              const uint2* range, float4* quad)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
-    const uint32_t child[2] = {__float_as_uint(node_ctr[i].w), __float_as_uint(node_half[i].w)};
-    for (int k = 0; k < 2; ++k) {
-        const PackedChild c = pack_child(n, leaf_size, node_ctr, node_half, range, child[k]);
-        PackedChild a = c, b;
-        if (c.cnt == 0u) {
-            a = pack_child(n, leaf_size, node_ctr, node_half, range, __float_as_uint(node_ctr[c.ref].w));
-            b = pack_child(n, leaf_size, node_ctr, node_half, range, __float_as_uint(node_half[c.ref].w));
-        } else {
-            b.ctr = b.half = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            b.ref = 0xffffffffu;
-            b.cnt = 0u;
+    PackedChild c[4];
+    c[0] = pack_child(n, leaf_size, node_ctr, node_half, range, __float_as_uint(node_ctr[i].w));
+    c[1] = pack_child(n, leaf_size, node_ctr, node_half, range, __float_as_uint(node_half[i].w));
+    int have = 2;
+    while (have < 4) {
+        int open = -1;
+        float most = -1.0f;
+        for (int k = 0; k < have; ++k) {
+            const float4 h = c[k].half;
+            const float area = h.x * h.y + h.y * h.z + h.z * h.x;
+            if (c[k].cnt == 0u && (open < 0 || area > most)) {
+                open = k;
+                most = area;
+            }
         }
+        if (open < 0) break;
+        const uint32_t ref = c[open].ref;
+        c[open] = pack_child(n, leaf_size, node_ctr, node_half, range, __float_as_uint(node_ctr[ref].w));
+        c[have++] = pack_child(n, leaf_size, node_ctr, node_half, range, __float_as_uint(node_half[ref].w));
+    }
+    for (int k = have; k < 4; ++k) {
+        c[k].ctr = c[k].half = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        c[k].ref = 0xffffffffu;
+        c[k].cnt = 0u;
+    }
+    for (int k = 0; k < 2; ++k) {
+        const PackedChild a = c[2 * k], b = c[2 * k + 1];
         float4* row = quad + 8 * (size_t)i + 4 * k;
         row[0] = make_float4(a.ctr.x, b.ctr.x, a.ctr.y, b.ctr.y);
         row[1] = make_float4(a.ctr.z, b.ctr.z, a.half.x, b.half.x);
