@@ -161,6 +161,16 @@ void Batch::release_scratch()
     }
 }
 
+void Batch::expect(uint32_t id, uint64_t paths)
+{
+    Slot* s = slot(id);
+    if (!s || s->settings.max_bounces <= 0 || cudaSetDevice(cfg_.device) != cudaSuccess) return;
+    const uint64_t bytes = s->scene.lists_bytes(), n = s->scene.view.n_sph, cap = budget_.cap();
+    if (bytes == 0 || paths < 4 * n * n || (cap && budget_.used() + bytes > cap / 2)) return;
+    s->scene.build_lists(&budget_, up_stream_, true);
+    (void)cudaEventRecord(uploaded_, up_stream_);
+}
+
 atx_status Batch::remove_scene(uint32_t id)
 {
     Slot* s = slot(id);

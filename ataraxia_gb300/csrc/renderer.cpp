@@ -140,12 +140,12 @@ bool SceneStore::lists_due(uint64_t paths)
     return due;
 }
 
-void SceneStore::build_lists(Budget* budget, cudaStream_t stream)
+void SceneStore::build_lists(Budget* budget, cudaStream_t stream, bool granted)
 {
     lists_tried = true;
     const uint32_t n = view.n_sph, nl = view.n_lights;
     const uint64_t lb = lb_bytes(nl, kBvhLightRes, kBvhLine), db = db_bytes(n, kBvhDirRes, kBvhLine);
-    if (budget && budget->cap()) return;   // what fitted the caller's budget still has to
+    if (!granted && budget && budget->cap()) return;   // what fitted the caller's budget still has to
     size_t free = 0, total = 0;
     if (cudaMemGetInfo(&free, &total) != cudaSuccess || (lbuf.bytes() + dbuf.bytes() < lb + db && (lb + db) > free / 16)) {
         (void)cudaGetLastError();
@@ -166,6 +166,13 @@ void SceneStore::build_lists(Budget* budget, cudaStream_t stream)
     }
     view.lb = lv;
     view.db = dv;
+}
+
+uint64_t SceneStore::lists_bytes() const
+{
+    const uint32_t n = view.n_sph, nl = view.n_lights;
+    if (!view.use_bvh || lists_tried || n > kDbMaxBvhSpheres || nl == 0 || nl > kLbMaxLights) return 0;
+    return lb_bytes(nl, kBvhLightRes, kBvhLine) + db_bytes(n, kBvhDirRes, kBvhLine);
 }
 
 uint32_t SceneStore::cells() const

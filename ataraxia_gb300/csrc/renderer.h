@@ -45,7 +45,10 @@ struct SceneStore {
     // set, which later buffers may need in full, or when the lists would take
     // more than a sixteenth of the device's free memory.
     bool lists_due(uint64_t paths);
-    void build_lists(Budget* budget, cudaStream_t stream);
+    // granted: the caller has seen to it that lists_bytes() fit its budget.
+    void build_lists(Budget* budget, cudaStream_t stream, bool granted = false);
+    // Device bytes of the lists this scene may get (0: none, or it has them).
+    uint64_t lists_bytes() const;
     uint64_t paths_seen = 0;    // since the upload, until the lists were tried
     bool lists_tried = false;
     uint64_t device_bytes() const

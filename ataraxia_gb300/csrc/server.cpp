@@ -55,6 +55,7 @@ public:
     }
     atx_status init() override { return b_.init(); }
     atx_status add(const atx_batch_scene& d, uint64_t, uint32_t* slot) override { return b_.add_scene(d, slot); }
+    void expect(uint32_t slot, uint64_t paths) override { b_.expect(slot, paths); }
     atx_status remove(uint32_t slot) override { return b_.remove_scene(slot); }
     atx_status set_spp(uint32_t slot, uint32_t spp) override { return b_.set_spp(slot, spp); }
     atx_status set_camera(uint32_t slot, const atx_camera& c) override { return b_.set_camera(slot, c); }
@@ -377,6 +378,7 @@ void Server::admit_locked()
             cv_done_.notify_all();
             continue;
         }
+        exec_->expect(slot, (uint64_t)j.desc.width * j.desc.height * j.target);
         j.slot = slot;
         j.state = ATX_JOB_ACTIVE;
         j.t_admit = now();

@@ -28,6 +28,8 @@ public:
     virtual atx_status init() = 0;
     // Makes a scene resident; its uploads do not wait for queued passes.
     virtual atx_status add(const atx_batch_scene& d, uint64_t bytes, uint32_t* slot) = 0;
+    // The slot's job is going to be rendered with this many paths.
+    virtual void expect(uint32_t, uint64_t) {}
     // Frees a slot after the work already queued (passes, read-backs).
     virtual atx_status remove(uint32_t slot) = 0;
     virtual atx_status set_spp(uint32_t slot, uint32_t spp) = 0;
