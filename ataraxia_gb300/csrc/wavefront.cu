@@ -1613,7 +1613,7 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
             for (int b = 0; b < bounces; ++b) {
                 if (inl && b >= kPathsFrom<IS>) {   // the late bounces in one persistent launch
                     // on half the resident blocks: the late bounces are a trickle of
-                    // paths, and the blocks stay resident until their pools drain,
+                    // paths, and the blocks stay resident until their paths end,
                     // holding slots the other lanes' kernels could use (+1%)
                     begin(kFamExtend);
                     k_paths<G><<<max(1, shape.blocks_extend / 2), kExtendThreads, 0, stream>>>(sc, ws, job, b);

@@ -78,13 +78,13 @@ struct BvhView {
     uint32_t root;
 };
 
-// Light buffer (Haines and Greenberg's light buffer, 1986) for the
-// brute-force sphere tables: for each point light a cube of directions around
+// Light buffer (Haines and Greenberg's light buffer, 1986) for the brute-force
+// sphere tables and LBVH scenes with lists (kDbMaxBvhSpheres): for each point light a cube of directions around
 // it, 6 faces of res x res cells, and for each cell the spheres that can
 // block a shadow ray towards that light whose origin, seen from the light,
 // lies in the cell (built by light_buffer.cu).  A shadow ray then tests the
 // spheres of one cell instead of the whole table.
-// Each cell is one 64-byte line of 16-bit words: word 0 the number of spheres
+// Each cell is one 64-byte line of 16-bit words (two for LBVH scenes): word 0 the number of spheres
 // listed (or kLbAll when they did not fit), words 1.. their indices in
 // ascending order, so the count and the first seven indices arrive in one
 // 16-byte load.
@@ -343,7 +343,9 @@ constexpr uint64_t kFusedSmallWork = 40000000;
 // thread (brute-force tables only; the wavefront for LBVH scenes).
 cudaError_t plan_launch(const SceneView& sc, int device, int threads, LaunchShape* out, int path_kernel = 0);
 
-// Enqueues one wave on stream: 2*max_bounces + 1 kernels plus a counter reset.
+// Enqueues one wave on stream: a counter reset and its kernels (one for a fused
+// wave, five with light and direction buffers on the brute-force tables, at most
+// 2*max_bounces + 3).
 // accum is W*H float4, image W*H uint32 (may be null when pack_frame == 0).
 // Returns the number of kernels launched through *launches.
 cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveState& ws, const WaveJob& job,

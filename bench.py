@@ -7,8 +7,8 @@ paths (one path = one pixel-sample).  Synthetic seeded scene (scenes.config1);
 the camera is set through the public API (atx_set_camera) as a caller would.
 
 Metric: Mpaths/s, whole job (N replicas on N GPUs, one process per GPU,
-`scaling: weak`).  The path state of a launch (four lanes of 8.3 Mi paths,
-about 1 GB each) is larger than L2, so every step streams its working set
+`scaling: weak`).  The path state of a launch (three lanes of 11 Mi paths,
+about 1.5 GB each) is larger than L2, so every step streams its working set
 through HBM; no explicit flush.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
@@ -351,7 +351,7 @@ def run_ours(args, dist: Dist):
     achieved_serial = alg_bytes / (launch_ms * 1e-3) / 1e9
     roofline = {
         "kernel": "one atx_render of the workload: k_primary, k_shadow (first-bounce pixel-light rays), "
-                  "k_first, k_shade (bounce 1), k_paths (bounces 2-7), k_accumulate per lane",
+                  "k_first, k_paths (bounces 1-7), k_accumulate per lane",
         "bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
         "frac": round(achieved / peak, 4) if peak else None,
         "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured copy bandwidth, burst)",
@@ -430,7 +430,7 @@ def run_ours(args, dist: Dist):
         "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded scenes.config1)",
         "config": {"workload": WORKLOAD_MEDIUM,
                    "paths_per_step": paths_step, "parallelism": f"replicas x{dist.world}",
-                   "l2": "working set > L2: four lanes of 8.3 Mi-path wave state (about 1 GB each) per launch"},
+                   "l2": "working set > L2: three lanes of 11 Mi-path wave state (about 1.5 GB each) per launch"},
         "mrays_per_s": round(mrays, 1),
         "rays_per_path": round(rays / (args.steps * paths_step), 4),
         "primary_hit_frac": round(shaded0 / (prof_steps * paths_step), 4),
@@ -933,7 +933,7 @@ def run_render_only(args, dist: Dist):
         sc = sc.with_resolution(args.width, args.height)
     from ataraxia_gb300 import _native as N
 
-    # the bench's own renderer: overlapped renders (4 lanes)
+    # the bench's own renderer: overlapped renders (3 lanes)
     r = atx.Renderer(device=dist.local_rank, bvh_threshold=args.bvh_threshold, bvh_leaf_size=args.bvh_leaf,
                      wave_paths=args.wave_paths, flags=N.FLAG_OVERLAP_RENDERS)
     r.on_resize(sc.width, sc.height)
