@@ -674,7 +674,7 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
     extern __shared__ float4 s_sph[];
     __shared__ uint32_t h_pid[kCap], h_id[kCap];
     __shared__ float h_t[kCap];
-    __shared__ uint32_t h_n;
+    __shared__ uint32_t h_n;   // where the next hit goes; its value is read through warp_push only
     const uint32_t n = ws.counters[2 * bounce];
     if (blockIdx.x * blockDim.x >= n) return;
     if (SMEM) stage_spheres(sc, s_sph);   // ends with a barrier
@@ -688,10 +688,14 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
     const bool last = bounce + 1 >= job.max_bounces;
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t base = blockIdx.x * blockDim.x;
+    // Hits in the list, counted by the barriers into every thread's register:
+    // a warp that is a turn ahead adds to h_n already while a late one still
+    // decides on this turn, so h_n itself would not be block-uniform.
+    uint32_t held = 0u;
     __syncthreads();
 
     for (;;) {   // ends: every round takes rays off the queue or hits off the list
-        while (base < n && h_n < blockDim.x) {   // block-uniform: base, h_n after the barrier
+        while (base < n && held < blockDim.x) {   // block-uniform
             const uint32_t idx = base + threadIdx.x;
             bool found = false;
             uint32_t pid = 0u;
@@ -721,9 +725,9 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
                 h_t[k] = tmin;
             }
             base += stride;
-            __syncthreads();
+            held += (uint32_t)__syncthreads_count(found);
         }
-        const uint32_t nh = h_n;
+        const uint32_t nh = held;
         if (nh == 0u) break;   // and the queue is done
         const uint32_t take = min(nh, blockDim.x);
         Shaded r{};
@@ -759,8 +763,9 @@ __global__ void __launch_bounds__(kExtendThreads, kExtendBlocksPerSm)
             }
         }
         push_shaded<false>(ws, qout, bounce, pid, r, o, d, thr, own, seed);
+        held = nh - take;
         __syncthreads();   // every thread has read its entry
-        if (threadIdx.x == 0) h_n = nh - take;
+        if (threadIdx.x == 0) h_n = held;
         __syncthreads();
     }
 }

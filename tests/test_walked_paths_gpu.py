@@ -49,3 +49,22 @@ def test_every_start_renders_the_same(po):
     for acc, st in out[1:]:
         assert st["shaded_first"] == out[0][1]["shaded_first"]
         assert bit_mismatches(acc, out[0][0]) == 0
+
+
+# waves large enough that k_bounce's blocks gather hits over several turns of their share of the queue
+# (bounces 1 to 3; a budget keeps the scene on its tree), against waves small enough to go without it;
+# repeated, since warps that disagreed about a turn would differ from run to run
+@pytest.mark.parametrize("spp", [24, 76])   # 5.5 M paths in one lane, 17.5 M in four
+def test_gathered_bounces_repeat(po, spp):
+    sc = _scene(1200, (640, 360), 5, 5)
+    view = po.view_for(sc)
+    want, _ = _frames(sc, view, spp, True, wave_paths=1 << 17, hbm_budget_bytes=8 << 30)
+    with Renderer(bvh_threshold=1, hbm_budget_bytes=8 << 30) as r:
+        r.on_resize(sc.width, sc.height)
+        r.set_scene(sc.spheres, sc.materials, sc.lights)
+        r.set_camera_matrices(np.array(view.inv_view), np.array(view.inv_proj), sc.camera_position)
+        r.set_settings(Settings(accumulation=True, skyLight=True, maxBounces=sc.max_bounces))
+        for _ in range(20):
+            r.reset_frame_index()
+            r.render_frames(spp)
+            assert bit_mismatches(r.get_accumulation().reshape(-1, 4), want) == 0
