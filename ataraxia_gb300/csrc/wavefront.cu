@@ -41,7 +41,7 @@ namespace atx {
 namespace {
 
 constexpr uint32_t kFull = 0xffffffffu;
-constexpr int kThreads = 256;
+constexpr int kThreads = kMaxBlockThreads;
 // k_first's and k_bounce's block: the shading code sets the register count.
 // 4 blocks of 256 threads per SM (64 registers) beat 6 of 192 (56 registers)
 // and 3 of 256 (80 registers) on the medium scene.
@@ -1534,7 +1534,7 @@ cudaError_t occupancy(uint32_t n_sph, int threads, size_t bytes, int* ext, int* 
 
 cudaError_t plan_launch(const SceneView& sc, int device, int threads, LaunchShape* out, int path_kernel)
 {
-    if (threads <= 0 || threads > kThreads) threads = kThreads;
+    threads = block_threads(threads);
     int sms = 0;
     cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;

@@ -338,7 +338,19 @@ constexpr uint32_t kFusedMaxSpp = 8;
 constexpr uint32_t kFusedSmallSpheres = 64;
 constexpr uint64_t kFusedSmallWork = 40000000;
 
-// Fills in grid sizes for this device and scene (occupancy-derived).
+// Threads per block of the primary and shadow kernels for a caller's count:
+// whole warps of at most 256 threads, since k_primary deals its tiles to warps
+// (a block without a whole warp would never come to an end of them, and the
+// rest of a part of one would take the next block's).
+constexpr int kMaxBlockThreads = 256;
+inline int block_threads(int asked)
+{
+    if (asked <= 0 || asked > kMaxBlockThreads) return kMaxBlockThreads;
+    return asked < 32 ? 32 : asked / 32 * 32;
+}
+
+// Fills in grid sizes for this device and scene (occupancy-derived); threads
+// goes through block_threads.
 // path_kernel: 0 by scene size, 1 the wavefront stages, 2 whole paths in one
 // thread (brute-force tables only; the wavefront for LBVH scenes).
 cudaError_t plan_launch(const SceneView& sc, int device, int threads, LaunchShape* out, int path_kernel = 0);

@@ -98,7 +98,8 @@ typedef struct atx_camera {
 typedef struct atx_config {
     int32_t device;            /* CUDA device ordinal */
     uint32_t wave_paths;       /* paths in flight per wave; 0 = autotuned default */
-    uint32_t threads;          /* threads per block; 0 = default */
+    uint32_t threads;          /* threads per block: whole warps are used, 32 to 256 (rounded down to a multiple
+                                  of 32, at least 32; 0 or more than 256 = 256) */
     uint32_t bvh_threshold;    /* sphere count at which the LBVH replaces the brute-force tables; 0 = 1025 */
     uint32_t bvh_leaf_size;    /* spheres per BVH leaf; 0 = 8, or what atx_autotune picks */
     uint32_t flags;            /* ATX_FLAG_* */
@@ -315,7 +316,7 @@ typedef struct atx_batch_stats {
 typedef struct atx_batch_tuning {
     uint32_t lanes;             /* concurrent streams, each with its own path state (default 8) */
     uint32_t lane_wave_paths;   /* path-state capacity of one lane, paths (default 16 Mi = 2.2 GB) */
-    uint32_t threads;           /* threads per CTA of the wavefront kernels (0 = per-kernel default) */
+    uint32_t threads;           /* threads per block, as atx_config.threads (0 = keep) */
     uint32_t bvh_threshold;     /* sphere count from which a scene uses its LBVH */
     uint32_t bvh_leaf_size;
     uint32_t primary_cache;     /* 1 (default): keep each scene's primary hits across passes; 2: trace them every pass */
