@@ -1,8 +1,9 @@
 """Late bounces (csrc/wavefront.cu k_paths): a lane carries a path to its end and takes the next of its warp's
 share.  Frames rendered in many lanes and one big wave equal those of small single waves bit for bit."""
+import numpy as np
 import pytest
 
-from helpers import bit_mismatches
+from helpers import bit_mismatches, oracle_render
 from ataraxia_gb300 import Camera, Renderer, Settings, scenes
 
 pytestmark = pytest.mark.gpu
@@ -35,3 +36,23 @@ def test_waves_of_any_size_render_the_same(n, res, spp, bounces, threshold, sky)
     want = _frames(sc, (1, spp), sky, bvh_threshold=threshold, wave_paths=4096)
     for _ in range(2):
         assert bit_mismatches(_frames(sc, (1, spp), sky, bvh_threshold=threshold), want) == 0
+
+
+# a ground sphere of radius 1000 under a few spheres, whose cell lists hold most of the table: 64 samples and up to
+# 15 bounces on two lanes, each frame sum against the oracle, over and over
+@pytest.mark.parametrize("bounces,sky", [(5, False), (15, True)])
+def test_ground_scene_repeats_bit_exact(po, bounces, sky):
+    sc = scenes.config0().with_resolution(640, 360)
+    sc.max_bounces = bounces
+    want, _, _ = oracle_render(sc, 64, sky=sky)
+    view = po.view_for(sc)
+    with Renderer() as r:
+        r.on_resize(sc.width, sc.height)
+        r.set_scene(sc.spheres, sc.materials, sc.lights)
+        r.set_camera_matrices(np.array(view.inv_view), np.array(view.inv_proj), sc.camera_position)
+        r.set_settings(Settings(accumulation=True, skyLight=sky, maxBounces=bounces))
+        for _ in range(20):
+            r.reset_frame_index()
+            r.render_frames(64)
+            assert bit_mismatches(r.get_accumulation().reshape(-1, 4), want) == 0
+            assert np.array_equal(r.get_image().reshape(-1), po.pack_rgba8(want, 64))
