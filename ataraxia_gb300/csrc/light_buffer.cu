@@ -234,7 +234,8 @@ __device__ __forceinline__ bool cap_meets(float3 axis, float ch, float sh, const
     return c.sb < 0.0f || dotf3(axis, c.v) >= c.dist * (ch * c.cb - sh * c.sb - 2e-5f);
 }
 
-constexpr uint32_t kFaceCap = 2048;   // caps a block keeps in shared memory (26 B each)
+constexpr uint32_t kFaceCap = 2048;   // caps a block keeps in shared memory
+constexpr size_t kCapBytes = sizeof(float4) + sizeof(float2) + sizeof(uint16_t);
 
 // The cell lists of both buffers: one block of 256 threads per (apex, cube
 // face, share of the face's tiles), the apexes the n_db spheres, then the
@@ -424,14 +425,17 @@ cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, cons
     k_cells_prep<<<cone_blocks + apex_l + (db ? 1u : 0u), 256, 0, stream>>>(sph, radius, n, lights, apex_l, res,
                                                                            cone_blocks, cones, dcap, reach);
     const uint32_t cap = n < kFaceCap ? (n + 7u) & ~7u : kFaceCap;
-    const size_t smem = cap * (sizeof(float4) + sizeof(float2) + sizeof(uint16_t));
+    const size_t smem = cap * kCapBytes;
     // few apexes: a face's tiles over several blocks (each repeats the face's
     // compaction), about four blocks per SM of the GPU in all
     const uint32_t blocks = (apex_d + apex_l) * 6u, shares = (tiles_for(res) + 7u) / 8u;
     const uint32_t want = (600u + blocks - 1u) / blocks;
     const dim3 grid(blocks, want < shares ? want : shares);
     const auto build = line_words == kBvhLine ? k_cells_build<kBvhLine> : k_cells_build<kLbLine>;
-    const cudaError_t e = cudaFuncSetAttribute(build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit belongs to the function on this device, not to this call: always
+    // the largest, so that a build on another thread never lowers it before this launch
+    const cudaError_t e =
+        cudaFuncSetAttribute(build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kFaceCap * kCapBytes));
     if (e != cudaSuccess) return e;
     build<<<grid, 256, smem, stream>>>(sph, radius, n, apex_d, reach, dline, lights, dcap, lline, res, cap, cones);
     if (lb) *lv = LightBufferView{lline, dcap, nl, res};
