@@ -1510,16 +1510,22 @@ size_t primary_smem(int mode, uint32_t n_sph, int threads, bool lists)
     return !lists && n_sph <= kCapSpheres ? n_sph * (sizeof(float4) + sizeof(float2)) : 0;
 }
 
+// Lets f be launched with any staged table.  The limit belongs to the function
+// on this device, not to a scene or a renderer: always the largest, so that
+// planning a smaller scene does not lower an earlier, larger one's.
+template <class F>
+cudaError_t allow_staged_table(F f)
+{
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemSphereCap);
+}
+
 template <int IS>
 cudaError_t occupancy(uint32_t n_sph, int threads, size_t bytes, int* ext, int* sh, int* pr)
 {
     if (bytes > 48 * 1024) {
-        const int b = (int)bytes;
-        const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        cudaError_t e = cudaFuncSetAttribute(k_bounce<IS>, a, b);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_shadow<IS, false>, a, b);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_shadow<IS, true>, a, b);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace<IS>, a, b);
+        cudaError_t e = allow_staged_table(k_bounce<IS>);
+        if (e == cudaSuccess) e = allow_staged_table(k_shadow<IS, false>);
+        if (e == cudaSuccess) e = allow_staged_table(k_shadow<IS, true>);
         if (e != cudaSuccess) return e;
     }
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ext, k_bounce<IS>, kExtendThreads, bytes);
@@ -1670,8 +1676,7 @@ cudaError_t enqueue_trace_nearest(const SceneView& sc, const float* origins, con
     cudaError_t e = cudaSuccess;
     with_mode(mode, [&](auto m) {
         constexpr int IS = decltype(m)::value;
-        if (bytes > 48 * 1024)
-            e = cudaFuncSetAttribute(k_trace<IS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (bytes > 48 * 1024) e = allow_staged_table(k_trace<IS>);
         if (e == cudaSuccess) k_trace<IS><<<g, kThreads, bytes, stream>>>(sc, origins, dirs, n, t_out, id_out);
     });
     if (e != cudaSuccess) return e;

@@ -2,6 +2,7 @@
 and rendered in turn or by threads of their own, do not lower one another's."""
 import threading
 
+import numpy as np
 import pytest
 
 from helpers import bit_mismatches
@@ -30,6 +31,22 @@ def _frames(r, spp=4):
     r.reset_frame_index()
     r.render_frames(spp)
     return r.get_accumulation().copy()
+
+
+# tables staged in 48 to 96 KB of shared memory (more lights than a light buffer holds, so the bounces test them whole):
+# the smaller scene is planned last, then the larger one renders and traces
+def test_a_smaller_scene_does_not_lower_a_larger_ones_limit():
+    big, small = _scene(5600, 70), _scene(3300, 70)
+    o = np.zeros((64, 3), dtype=np.float32)
+    d = np.tile(np.array([[0.6, 0.0, 0.8]], dtype=np.float32), (64, 1))
+    with Renderer(bvh_threshold=1 << 30) as a, Renderer(bvh_threshold=1 << 30) as b:
+        _set(a, big)
+        want, hit = _frames(a), a.trace_nearest(o, d)
+        _set(b, small)
+        _frames(b)
+        b.trace_nearest(o, d)
+        assert bit_mismatches(_frames(a), want) == 0
+        assert np.array_equal(a.trace_nearest(o, d)[1], hit[1])
 
 
 # light buffers built by several threads at once, of tables above and below what their builds may use without a raised
