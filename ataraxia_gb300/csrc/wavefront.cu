@@ -1526,6 +1526,9 @@ cudaError_t occupancy(uint32_t n_sph, int threads, size_t bytes, int* ext, int* 
         cudaError_t e = allow_staged_table(k_bounce<IS>);
         if (e == cudaSuccess) e = allow_staged_table(k_shadow<IS, false>);
         if (e == cudaSuccess) e = allow_staged_table(k_shadow<IS, true>);
+        if constexpr (IS == kIsSmem) {
+            if (e == cudaSuccess) e = allow_staged_table(k_fused<IS>);
+        }
         if (e != cudaSuccess) return e;
     }
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ext, k_bounce<IS>, kExtendThreads, bytes);

@@ -49,6 +49,16 @@ def test_a_smaller_scene_does_not_lower_a_larger_ones_limit():
         assert np.array_equal(a.trace_nearest(o, d)[1], hit[1])
 
 
+# whole paths in one thread over such a table
+def test_fused_paths_take_a_large_table():
+    sc = _scene(3300, 70)
+    with Renderer(bvh_threshold=1 << 30) as r:
+        _set(r, sc)
+        want = _frames(r)
+        r.set_tuning(path_kernel=2)
+        assert bit_mismatches(_frames(r), want) == 0
+
+
 # light buffers built by several threads at once, of tables above and below what their builds may use without a raised
 # limit
 def test_threads_build_cell_lists_of_different_sizes():
