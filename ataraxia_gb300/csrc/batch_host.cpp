@@ -113,6 +113,7 @@ atx_status Batch::add_scene(const atx_batch_scene& d, uint32_t* id)
     s->prim.use_stream_order(&order_);
     s->dirs.use_stream_order(&order_);
     s->scene.cell_res = cell_res_;
+    s->scene.lists_on = lists_;
     // on the upload stream: a pass running on the batch stream is not waited for
     ATX_TRY(s->scene.upload(d.spheres, d.n_spheres, d.materials, d.n_materials, d.lights, d.n_lights, &budget_,
                             up_stream_));
@@ -164,7 +165,7 @@ void Batch::release_scratch()
 void Batch::expect(uint32_t id, uint64_t paths)
 {
     Slot* s = slot(id);
-    if (!s || s->settings.max_bounces <= 0 || cudaSetDevice(cfg_.device) != cudaSuccess) return;
+    if (!s || s->settings.max_bounces <= 1 || cudaSetDevice(cfg_.device) != cudaSuccess) return;
     const uint64_t bytes = s->scene.lists_bytes(), n = s->scene.view.n_sph, cap = budget_.cap();
     if (bytes == 0 || paths < 4 * n * n || (cap && budget_.used() + bytes > cap / 2)) return;
     s->scene.build_lists(&budget_, up_stream_, true);
@@ -261,7 +262,7 @@ atx_status Batch::autotune(uint32_t passes, atx_batch_tuning* chosen)
     if (!passes) passes = 2;
     // the trials are passes over the same scenes: lists they would get on the way come first
     for (auto& p : slots_)
-        if (p && lists_ && p->scene.lists_due(16ull * kDbMaxBvhSpheres * kDbMaxBvhSpheres)) {
+        if (p && lists_ && p->scene.lists_possible(p->settings.max_bounces)) {
             p->scene.build_lists(&budget_, up_stream_);
             ATX_CUDA(cudaEventRecord(uploaded_, up_stream_));
         }
@@ -372,8 +373,8 @@ atx_status Batch::run(cudaEvent_t done)
         const uint64_t px = (uint64_t)s->w * s->h;
         const uint64_t p = px * s->spp_next;
         paths += p;
-        if (lists_ && s->settings.max_bounces > 0 && s->scene.lists_due(p)) {
-            s->scene.build_lists(&budget_, up_stream_);
+        if (s->scene.lists_due(p, s->settings.max_bounces)) {
+            ATX_TRY(s->scene.lists_step(p, &budget_, up_stream_, stream_));
             ATX_CUDA(cudaEventRecord(uploaded_, up_stream_));
         }
         const uint64_t want = (p + tuning_.lane_wave_paths - 1) / tuning_.lane_wave_paths;

@@ -30,7 +30,7 @@ atx_status SceneStore::upload(const atx_sphere* s, uint32_t n, const atx_materia
 {
     if ((n && !s) || (nm && !m) || (nl && !l)) return fail(ATX_ERR_INVALID_ARG, "set_scene: null array");
     if (n > 0 && nm == 0) return fail(ATX_ERR_INVALID_ARG, "set_scene: spheres need at least one material");
-    for (DeviceBuffer* b : {&this->sph, &sph_mat, &sph_rad, &mat, &lights, &bvh, &lbuf, &dbuf})
+    for (DeviceBuffer* b : {&this->sph, &sph_mat, &sph_rad, &mat, &lights, &bvh, &lbuf, &dbuf, &rays})
         b->use_stream_order(order);
 
     std::vector<float4> sph(n);
@@ -80,6 +80,7 @@ atx_status SceneStore::upload(const atx_sphere* s, uint32_t n, const atx_materia
     view.n_lights = nl;
     view.light_mod = fastmod_multiplier(nl);
     paths_seen = 0;
+    look_at = 2 * (uint64_t)n * n;
     lists_tried = false;
 
     const uint32_t thr = bvh_threshold ? bvh_threshold : kDefaultBvhThreshold;
@@ -91,8 +92,16 @@ atx_status SceneStore::upload(const atx_sphere* s, uint32_t n, const atx_materia
                             bvh.bytes(), &bv, stream));
         view.bvh = bv;
         view.use_bvh = 1;
+        if (lists_on && lists_possible(2) && !(budget && budget->cap())) {   // lists may follow
+            ATX_TRY(rays.ensure(sizeof(unsigned long long), budget, "ray total"));
+            ATX_CUDA(cudaMemsetAsync(rays.get(), 0, sizeof(unsigned long long), stream));
+            view.rays = rays.as<unsigned long long>();
+        } else {
+            rays.reset();
+        }
     } else {
         bvh.reset();
+        rays.reset();
     }
     ATX_TRY(build_cells(budget, stream));
     ATX_CUDA(cudaStreamSynchronize(stream));
@@ -124,20 +133,53 @@ atx_status SceneStore::build_cells(Budget* budget, cudaStream_t stream)
     return ATX_OK;
 }
 
-bool SceneStore::lists_due(uint64_t paths)
+bool SceneStore::lists_possible(int32_t bounces) const
 {
-    const uint64_t n = view.n_sph;
-    if (!view.use_bvh || lists_tried || n > kDbMaxBvhSpheres || view.n_lights == 0 || view.n_lights > kLbMaxLights)
-        return false;
-    // The build takes 7.5 ms at 4,096 spheres, 39 at 8,000, and a path over the
-    // lists instead of the tree saves 0.17 and 0.24 ns there (16 samples of
-    // 1280x720 pixels), so it pays after about 2 n^2 paths.
+    // without a second bounce there is no extension ray to look up
+    return view.use_bvh && bounces > 1 && !lists_tried && view.n_sph <= kDbMaxBvhSpheres &&
+           view.n_lights != 0 && view.n_lights <= kLbMaxLights;
+}
+
+bool SceneStore::lists_due(uint64_t paths, int32_t bounces)
+{
+    if (!lists_on || !lists_possible(bounces)) return false;
     // The call at hand counts for an eighth of its paths: a scene uploaded for
     // every render would build its lists each time (1,471 clustered spheres, 4
     // samples of 2560x1440 pixels: 1.13 against 0.79 ms).
-    const bool due = paths_seen + paths / 8 >= 2 * n * n;
+    const bool due = paths_seen + paths / 8 >= look_at;
     paths_seen += paths;
     return due;
+}
+
+atx_status SceneStore::lists_step(uint64_t paths, Budget* budget, cudaStream_t stream, cudaStream_t work)
+{
+    const uint64_t n = view.n_sph;
+    if (!rays.get()) {   // a budget was set
+        lists_tried = true;
+        return ATX_OK;
+    }
+    // The build takes 7.5 ms at 4,096 spheres and 39 at 8,000, 0.45 and 0.61
+    // ns a pair; a ray looked up instead of walked saves 0.4 to 0.5 ns (16
+    // samples of 1280x720 pixels, 0.41 and 0.50 rays a path), so the build is
+    // worth n^2 rays.  It is started at 2 n^2 paths if they traced a quarter
+    // of that, as paths that see the scene do; otherwise looked at again when
+    // they have doubled (8,000 spheres in clusters, of which 0.023 rays a path
+    // come: 11 n^2; a camera that looks past the scene: never).  Before a
+    // first render nothing is known, but one of 16 n^2 paths is worth the
+    // build when one path in sixteen traces a ray.
+    const uint64_t before = paths_seen - paths;
+    if (before) {
+        unsigned long long r = 0;
+        ATX_CUDA(cudaMemcpyAsync(&r, rays.get(), sizeof(r), cudaMemcpyDeviceToHost, work));
+        ATX_CUDA(cudaStreamSynchronize(work));
+        const double rays_per_path = (double)r / (double)before;
+        if (rays_per_path * (double)(before + paths / 8) < 0.25 * (double)n * (double)n) {
+            look_at = 2 * before;
+            return ATX_OK;
+        }
+    }
+    build_lists(budget, stream);
+    return ATX_OK;
 }
 
 void SceneStore::build_lists(Budget* budget, cudaStream_t stream, bool granted)
@@ -170,9 +212,8 @@ void SceneStore::build_lists(Budget* budget, cudaStream_t stream, bool granted)
 
 uint64_t SceneStore::lists_bytes() const
 {
-    const uint32_t n = view.n_sph, nl = view.n_lights;
-    if (!view.use_bvh || lists_tried || n > kDbMaxBvhSpheres || nl == 0 || nl > kLbMaxLights) return 0;
-    return lb_bytes(nl, kBvhLightRes, kBvhLine) + db_bytes(n, kBvhDirRes, kBvhLine);
+    if (!lists_possible(2)) return 0;
+    return lb_bytes(view.n_lights, kBvhLightRes, kBvhLine) + db_bytes(view.n_sph, kBvhDirRes, kBvhLine);
 }
 
 uint32_t SceneStore::cells() const
@@ -672,9 +713,9 @@ atx_status Renderer::render(uint32_t spp)
         capacity = (uint32_t)std::min<uint64_t>(want, kDefaultWavePaths);
     }
     const int32_t bounces = settings_.max_bounces;
-    if (bounces > 0 && scene_.lists_due(px * spp)) {
+    if (scene_.lists_due(px * spp, bounces)) {
         ATX_TRY(join());
-        scene_.build_lists(&budget_, stream_);
+        ATX_TRY(scene_.lists_step(px * spp, &budget_, stream_, stream_));
         stream_dirty_ = true;
     }
     if (!settings_.accumulation) frame_ = 1;
@@ -1008,7 +1049,7 @@ atx_status Renderer::autotune(uint32_t spp, uint32_t passes, bool use_cache, atx
         }
     }
     // the trials are renders of one scene: lists it would get on the way come first
-    if (scene_.lists_due(16ull * kDbMaxBvhSpheres * kDbMaxBvhSpheres)) {
+    if (scene_.lists_possible(settings_.max_bounces)) {
         ATX_TRY(join());
         scene_.build_lists(&budget_, stream_);
         stream_dirty_ = true;

@@ -14,7 +14,7 @@ namespace atx {
 // Device-resident scene: sphere table (float4 centre + radius^2), clamped
 // material ids, radii (for BVH boxes), shading tables and the optional LBVH.
 struct SceneStore {
-    DeviceBuffer sph, sph_mat, sph_rad, mat, lights, bvh, lbuf, dbuf;
+    DeviceBuffer sph, sph_mat, sph_rad, mat, lights, bvh, lbuf, dbuf, rays;
     SceneView view{};
     uint32_t bvh_threshold = 0;
     uint32_t bvh_leaf = 0;
@@ -38,23 +38,31 @@ struct SceneStore {
     atx_status build_cells(Budget* budget, cudaStream_t stream);
     // Light and direction buffers for an LBVH scene of up to kDbMaxBvhSpheres
     // spheres, on top of its tree.  Every pair of spheres is looked at, so they
-    // are built only for a scene that goes on being rendered: lists_due counts
-    // the paths of each render and says, before it, when those so far would
-    // have paid for the build; a scene rendered once, or uploaded for every render, keeps
-    // to the tree.  build_lists leaves the scene on the tree when a budget is
-    // set, which later buffers may need in full, or when the lists would take
-    // more than a sixteenth of the device's free memory.
-    bool lists_due(uint64_t paths);
+    // are built only for a scene that goes on being rendered and whose paths
+    // trace rays that the lists would save: a scene rendered once, uploaded for
+    // every render, rendered without bounces after the first or seen by a camera
+    // that looks past it keeps to the tree.  It also does when a budget is set,
+    // which later buffers may need in full, or when the lists would take more
+    // than a sixteenth of the device's free memory.
+    // Before each render: lists_due counts its paths and says when lists_step
+    // has something to do, which is to wait for the renders queued on `work` and
+    // look at the rays they traced, and to build the lists on stream when they pay.
+    bool lists_due(uint64_t paths, int32_t bounces);
+    atx_status lists_step(uint64_t paths, Budget* budget, cudaStream_t stream, cudaStream_t work);
+    // Whether the lists may still come.
+    bool lists_possible(int32_t bounces) const;
     // granted: the caller has seen to it that lists_bytes() fit its budget.
     void build_lists(Budget* budget, cudaStream_t stream, bool granted = false);
     // Device bytes of the lists this scene may get (0: none, or it has them).
     uint64_t lists_bytes() const;
-    uint64_t paths_seen = 0;    // since the upload, until the lists were tried
-    bool lists_tried = false;
+    bool lists_on = true;         // renders count towards lists (a server decides when it admits a job)
+    uint64_t paths_seen = 0;      // since the upload, until the lists were tried
+    uint64_t look_at = 0;         // paths at which the rays are looked at next
+    bool lists_tried = false;     // built or given up
     uint64_t device_bytes() const
     {
         return sph.bytes() + sph_mat.bytes() + sph_rad.bytes() + mat.bytes() + lights.bytes() + bvh.bytes() +
-               lbuf.bytes() + dbuf.bytes();
+               lbuf.bytes() + dbuf.bytes() + rays.bytes();
     }
 };
 

@@ -1144,17 +1144,20 @@ __global__ void __launch_bounds__(kThreads) k_accumulate(WaveState ws, WaveJob j
 {
     const uint32_t stride = gridDim.x * blockDim.x;
     const float fpack = __uint2float_rn(job.pack_frame);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && ws.totals) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (ws.totals || job.rays)) {
         unsigned long long ext = 0, sh = 0;
         for (int b = 0; b < job.max_bounces; ++b) {
             if (b > 0) ext += ws.counters[2 * b];
             sh += ws.counters[2 * b + 1];
         }
         if (job.max_bounces > 0) ext += ws.counters[2 * ((uint32_t)job.max_bounces + 1u) + 3u];
-        atomicAdd(&ws.totals[0], ext);
-        atomicAdd(&ws.totals[1], sh);
+        if (job.rays) atomicAdd(job.rays, ext + sh);
+        if (ws.totals) {
+            atomicAdd(&ws.totals[0], ext);
+            atomicAdd(&ws.totals[1], sh);
+        }
         // every sample of a hit pixel is shaded at the first bounce
-        if (job.max_bounces > 0)
+        if (ws.totals && job.max_bounces > 0)
             atomicAdd(&ws.totals[2],
                       (unsigned long long)ws.counters[2 * ((uint32_t)job.max_bounces + 1u)] * job.spp);
     }
@@ -1569,6 +1572,7 @@ cudaError_t enqueue_wave(const SceneView& sc, const CameraView& cam, const WaveS
 {
     WaveJob job = wave;
     job.spp_div = fastmod_multiplier(job.spp);
+    job.rays = sc.rays;
     uint32_t nl = 0;
     const size_t sm = shape.smem_spheres;
     const int bounces = job.max_bounces;

@@ -167,6 +167,7 @@ struct SceneView {
     LightBufferView lb;       // shadow-ray cells (lb.n_lights 0: none)
     DirBufferView db;         // extension-ray cells (db.n 0: none; with the LBVH both or neither)
     uint64_t light_mod;       // fastmod_multiplier(n_lights): x % n_lights by multiplication
+    unsigned long long* rays; // device total of the rays traced after the primary ones (null: not kept)
 };
 
 // x % d for d >= 1 by two multiplications (Lemire, Kaser and Kurz, "Faster
@@ -284,6 +285,7 @@ struct WaveJob {
     // clears it).
     int32_t fresh;
     uint64_t spp_div;         // fastmod_multiplier(spp), set by enqueue_wave: x / spp by multiplication
+    unsigned long long* rays; // the scene's (SceneView), set by enqueue_wave
 };
 
 // Whether the first bounce's shadow rays are traced once per (pixel, light)

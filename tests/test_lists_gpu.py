@@ -98,3 +98,32 @@ def test_lists_in_a_batch_and_after_a_new_scene():
             got = r.get_accumulation().reshape(-1, 4)
             want, _ = _render(s, (1, frames, 1), False, bvh_threshold=1 << 30)
             assert bit_mismatches(got, want[-1]) == 0
+
+
+def test_no_lists_for_rays_that_are_not_traced():
+    n = 1100
+    sc = _scene("open", n, 4)
+    frames = 2 * n * n // sc.pixels + 1
+    cam = Camera(sc.fov, sc.near, sc.far, sc.camera_position, sc.camera_direction)
+    away = Camera(sc.fov, sc.near, sc.far, sc.camera_position, tuple(-np.array(sc.camera_direction)))
+    with Renderer(wave_paths=1 << 18) as r:   # little path state beside the lists
+        r.on_resize(sc.width, sc.height)
+        r.set_scene(sc.spheres, sc.materials, sc.lights)
+        r.set_settings(Settings(maxBounces=1))
+        r.set_camera(cam)
+        for _ in range(3):                       # no bounce that would leave a sphere
+            r.render_frames(frames)
+        assert r.stats()["device_bytes"] < n * 300_000
+        r.set_settings(Settings(maxBounces=sc.max_bounces))
+        r.set_camera(away)
+        for _ in range(6):                       # a camera that sees no sphere
+            r.render_frames(frames)
+        assert r.stats()["device_bytes"] < n * 300_000
+        r.set_camera(cam)
+        r.reset_frame_index()
+        for _ in range(12):                      # and one that turns to them
+            r.render_frames(frames)
+        assert r.stats()["device_bytes"] > n * 300_000
+        got = r.get_accumulation().reshape(-1, 4)
+    want, _ = _render(sc, (frames,) * 12, False, bvh_threshold=1 << 30)
+    assert bit_mismatches(got, want[-1]) == 0
