@@ -168,7 +168,7 @@ void Batch::expect(uint32_t id, uint64_t paths)
     if (!s || s->settings.max_bounces <= 1 || cudaSetDevice(cfg_.device) != cudaSuccess) return;
     const uint64_t bytes = s->scene.lists_bytes(), n = s->scene.view.n_sph, cap = budget_.cap();
     if (bytes == 0 || paths < 4 * n * n || (cap && budget_.used() + bytes > cap / 2)) return;
-    s->scene.build_lists(&budget_, up_stream_, true);
+    s->scene.build_lists(&budget_, up_stream_, ~uint64_t(0), true);
     (void)cudaEventRecord(uploaded_, up_stream_);
 }
 

@@ -238,8 +238,8 @@ constexpr uint32_t kFaceCap = 2048;   // caps a block keeps in shared memory
 constexpr size_t kCapBytes = sizeof(float4) + sizeof(float2) + sizeof(uint16_t);
 
 // The cell lists of both buffers: one block of 256 threads per (apex, cube
-// face, share of the face's tiles), the apexes the n_db spheres, then the
-// nl lights.
+// face, share of the face's tiles), the apexes n_db spheres from db_first on,
+// then the nl lights.
 //
 // First the block keeps the spheres whose caps meet the face's bounding cone
 // (its corners lie acos(1/sqrt 3) from the face axis), in index order, with
@@ -258,7 +258,8 @@ constexpr size_t kCapBytes = sizeof(float4) + sizeof(float2) + sizeof(uint16_t);
 // the fly).
 template <uint32_t LINE>
 __global__ void __launch_bounds__(256) k_cells_build(const float4* __restrict__ sph, const float* __restrict__ rad,
-                                                     uint32_t n, uint32_t n_db, const float* __restrict__ reach,
+                                                     uint32_t n, uint32_t db_first, uint32_t n_db,
+                                                     const float* __restrict__ reach,
                                                      uint16_t* db_line, const DevLight* __restrict__ lights,
                                                      const float* __restrict__ dcap, uint16_t* lb_line, uint32_t res,
                                                      uint32_t face_cap, Cones cones)
@@ -277,11 +278,12 @@ __global__ void __launch_bounds__(256) k_cells_build(const float4* __restrict__ 
     float rho, e1, e2;
     uint16_t* line;
     if (apex < n_db) {
-        const float4 s = sph[apex];
+        const uint32_t i = db_first + apex;
+        const float4 s = sph[i];
         o = make_float3(s.x, s.y, s.z);
-        rho = reach[apex];
+        rho = reach[i];
         e1 = 0.0f, e2 = rho;
-        line = db_line + (size_t)apex * cells_for(res) * LINE;
+        line = db_line + (size_t)i * cells_for(res) * LINE;
     } else {
         const uint32_t l = apex - n_db;
         o = make_float3(lights[l].pos[0], lights[l].pos[1], lights[l].pos[2]);
@@ -397,7 +399,8 @@ uint64_t db_bytes(uint32_t n, uint32_t res, uint32_t line_words)
 
 cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, const DevLight* lights, uint32_t nl,
                         uint32_t res, uint32_t line_words, void* lbuf, uint64_t lbytes, LightBufferView* lv,
-                        void* dbuf, uint64_t dbytes, DirBufferView* dv, cudaStream_t stream)
+                        void* dbuf, uint64_t dbytes, DirBufferView* dv, cudaStream_t stream, uint32_t db_first,
+                        uint32_t db_count)
 {
     const bool lb = lbuf != nullptr, db = dbuf != nullptr;
     if (!lb && !db) return cudaSuccess;
@@ -405,7 +408,8 @@ cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, cons
         (line_words != kLbLine && line_words != kBvhLine))
         return cudaErrorInvalidValue;
     if (lb && (nl == 0 || nl > kLbMaxLights || lbytes < lb_bytes(nl, res, line_words))) return cudaErrorInvalidValue;
-    if (db && (n > kDbMaxBvhSpheres || dbytes < db_bytes(n, res, line_words))) return cudaErrorInvalidValue;
+    if (db && (n > kDbMaxBvhSpheres || dbytes < db_bytes(n, res, line_words) || db_first >= n))
+        return cudaErrorInvalidValue;
     const uint64_t row = (uint64_t)cells_for(res) * line_words * sizeof(uint16_t);
     uint16_t* lline = static_cast<uint16_t*>(lbuf);
     uint16_t* dline = static_cast<uint16_t*>(dbuf);
@@ -420,7 +424,8 @@ cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, cons
         end = reinterpret_cast<unsigned char*>(reach) + up(n * sizeof(float));
     }
     const Cones cones = carve_cones(end, res);
-    const uint32_t apex_l = lb ? nl : 0u, apex_d = db ? n : 0u;
+    const uint32_t apex_l = lb ? nl : 0u, apex_d = !db ? 0u : db_count < n - db_first ? db_count : n - db_first;
+    if (apex_l + apex_d == 0u) return cudaErrorInvalidValue;
     const uint32_t cone_blocks = (6u * tiles_for(res) + 7u) / 8u;
     k_cells_prep<<<cone_blocks + apex_l + (db ? 1u : 0u), 256, 0, stream>>>(sph, radius, n, lights, apex_l, res,
                                                                            cone_blocks, cones, dcap, reach);
@@ -437,7 +442,7 @@ cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, cons
     const cudaError_t e =
         cudaFuncSetAttribute(build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kFaceCap * kCapBytes));
     if (e != cudaSuccess) return e;
-    build<<<grid, 256, smem, stream>>>(sph, radius, n, apex_d, reach, dline, lights, dcap, lline, res, cap, cones);
+    build<<<grid, 256, smem, stream>>>(sph, radius, n, db_first, apex_d, reach, dline, lights, dcap, lline, res, cap, cones);
     if (lb) *lv = LightBufferView{lline, dcap, nl, res};
     if (db) *dv = DirBufferView{dline, reach, n, res};
     return cudaGetLastError();

@@ -23,9 +23,11 @@ uint64_t db_bytes(uint32_t n, uint32_t res, uint32_t line_words = kLbLine);
 //   kLbMaxSpheres) into lbuf (lb_bytes() of device memory; null: none), *lv
 //   its view;
 //   the direction buffer (n <= kDbMaxBvhSpheres) into dbuf (db_bytes(); null:
-//   none), *dv its view.
+//   none), *dv its view: the cells of spheres db_first.. db_first + db_count - 1
+//   of it, so that a large one can be built over several calls.
 cudaError_t cells_build(const float4* sph, const float* radius, uint32_t n, const DevLight* lights, uint32_t nl,
                         uint32_t res, uint32_t line_words, void* lbuf, uint64_t lbytes, LightBufferView* lv,
-                        void* dbuf, uint64_t dbytes, DirBufferView* dv, cudaStream_t stream);
+                        void* dbuf, uint64_t dbytes, DirBufferView* dv, cudaStream_t stream, uint32_t db_first = 0,
+                        uint32_t db_count = ~0u);
 
 }  // namespace atx

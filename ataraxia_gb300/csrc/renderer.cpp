@@ -81,7 +81,10 @@ atx_status SceneStore::upload(const atx_sphere* s, uint32_t n, const atx_materia
     view.light_mod = fastmod_multiplier(nl);
     paths_seen = 0;
     look_at = 2 * (uint64_t)n * n;
+    rays_per_path = 0.4;
     lists_tried = false;
+    lists_lb = LightBufferView{};
+    lists_db = DirBufferView{};
 
     const uint32_t thr = bvh_threshold ? bvh_threshold : kDefaultBvhThreshold;
     if (n >= thr && n > 1) {
@@ -136,13 +139,15 @@ atx_status SceneStore::build_cells(Budget* budget, cudaStream_t stream)
 bool SceneStore::lists_possible(int32_t bounces) const
 {
     // without a second bounce there is no extension ray to look up
-    return view.use_bvh && bounces > 1 && !lists_tried && view.n_sph <= kDbMaxBvhSpheres &&
+    const bool building = lists_db.n != 0 && view.db.n == 0;
+    return view.use_bvh && bounces > 1 && (!lists_tried || building) && view.n_sph <= kDbMaxBvhSpheres &&
            view.n_lights != 0 && view.n_lights <= kLbMaxLights;
 }
 
 bool SceneStore::lists_due(uint64_t paths, int32_t bounces)
 {
     if (!lists_on || !lists_possible(bounces)) return false;
+    if (lists_tried) return true;   // being built
     // The call at hand counts for an eighth of its paths: a scene uploaded for
     // every render would build its lists each time (1,471 clustered spheres, 4
     // samples of 2560x1440 pixels: 1.13 against 0.79 ms).
@@ -154,65 +159,78 @@ bool SceneStore::lists_due(uint64_t paths, int32_t bounces)
 atx_status SceneStore::lists_step(uint64_t paths, Budget* budget, cudaStream_t stream, cudaStream_t work)
 {
     const uint64_t n = view.n_sph;
-    if (!rays.get()) {   // a budget was set
-        lists_tried = true;
-        return ATX_OK;
-    }
-    // The build takes 7.5 ms at 4,096 spheres and 39 at 8,000, 0.45 and 0.61
-    // ns a pair; a ray looked up instead of walked saves 0.4 to 0.5 ns (16
-    // samples of 1280x720 pixels, 0.41 and 0.50 rays a path), so the build is
-    // worth n^2 rays.  It is started at 2 n^2 paths if they traced a quarter
-    // of that, as paths that see the scene do; otherwise looked at again when
-    // they have doubled (8,000 spheres in clusters, of which 0.023 rays a path
-    // come: 11 n^2; a camera that looks past the scene: never).  Before a
-    // first render nothing is known, but one of 16 n^2 paths is worth the
-    // build when one path in sixteen traces a ray.
-    const uint64_t before = paths_seen - paths;
-    if (before) {
-        unsigned long long r = 0;
-        ATX_CUDA(cudaMemcpyAsync(&r, rays.get(), sizeof(r), cudaMemcpyDeviceToHost, work));
-        ATX_CUDA(cudaStreamSynchronize(work));
-        const double rays_per_path = (double)r / (double)before;
-        if (rays_per_path * (double)(before + paths / 8) < 0.25 * (double)n * (double)n) {
-            look_at = 2 * before;
+    if (!lists_tried) {
+        if (!rays.get()) {   // a budget was set
+            lists_tried = true;
             return ATX_OK;
         }
+        // The build takes 7.5 ms at 4,096 spheres and 39 at 8,000, 0.45 and 0.61
+        // ns a pair; a ray looked up instead of walked saves 0.4 to 0.5 ns (16
+        // samples of 1280x720 pixels, 0.41 and 0.50 rays a path), so the build is
+        // worth n^2 rays.  It is started at 2 n^2 paths if they traced a quarter
+        // of that, as paths that see the scene do; otherwise looked at again when
+        // they have doubled (8,000 spheres in clusters, of which 0.023 rays a path
+        // come: 11 n^2; a camera that looks past the scene: never).  Before a
+        // first render nothing is known, but one of 16 n^2 paths is worth the
+        // build when one path in sixteen traces a ray.
+        const uint64_t before = paths_seen - paths;
+        if (before) {
+            unsigned long long r = 0;
+            ATX_CUDA(cudaMemcpyAsync(&r, rays.get(), sizeof(r), cudaMemcpyDeviceToHost, work));
+            ATX_CUDA(cudaStreamSynchronize(work));
+            rays_per_path = (double)r / (double)before;
+            if (rays_per_path * (double)(before + paths / 8) < 0.25 * (double)n * (double)n) {
+                look_at = 2 * before;
+                return ATX_OK;
+            }
+        }
     }
-    build_lists(budget, stream);
+    // A render adds to the build what takes about as long as its own rays' walks
+    // (1 ns each), and at least some 2 ms, so that no single call waits for all of it.
+    build_lists(budget, stream, std::max<uint64_t>(4u << 20, (uint64_t)(2.0 * rays_per_path * (double)paths)));
     return ATX_OK;
 }
 
-void SceneStore::build_lists(Budget* budget, cudaStream_t stream, bool granted)
+void SceneStore::build_lists(Budget* budget, cudaStream_t stream, uint64_t pairs, bool granted)
 {
-    lists_tried = true;
     const uint32_t n = view.n_sph, nl = view.n_lights;
     const uint64_t lb = lb_bytes(nl, kBvhLightRes, kBvhLine), db = db_bytes(n, kBvhDirRes, kBvhLine);
-    if (!granted && budget && budget->cap()) return;   // what fitted the caller's budget still has to
-    size_t free = 0, total = 0;
-    if (cudaMemGetInfo(&free, &total) != cudaSuccess || (lbuf.bytes() + dbuf.bytes() < lb + db && (lb + db) > free / 16)) {
-        (void)cudaGetLastError();
-        return;
+    bool ok = true;
+    if (!lists_tried) {
+        lists_tried = true;
+        lists_next = 0;
+        if (!granted && budget && budget->cap()) return;   // what fitted the caller's budget still has to
+        size_t free = 0, total = 0;
+        if (cudaMemGetInfo(&free, &total) != cudaSuccess ||
+            (lbuf.bytes() + dbuf.bytes() < lb + db && (lb + db) > free / 16)) {
+            (void)cudaGetLastError();
+            return;
+        }
+        ok = lbuf.ensure(lb, budget, "light buffer") == ATX_OK && dbuf.ensure(db, budget, "direction buffer") == ATX_OK &&
+             cells_build(view.sph, sph_rad.as<float>(), n, view.lights, nl, kBvhLightRes, kBvhLine, lbuf.get(),
+                         lbuf.bytes(), &lists_lb, nullptr, 0, nullptr, stream) == cudaSuccess;
     }
-    LightBufferView lv{};
-    DirBufferView dv{};
-    if (lbuf.ensure(lb, budget, "light buffer") != ATX_OK || dbuf.ensure(db, budget, "direction buffer") != ATX_OK ||
-        cells_build(view.sph, sph_rad.as<float>(), n, view.lights, nl, kBvhLightRes, kBvhLine, lbuf.get(),
-                    lbuf.bytes(), &lv, nullptr, 0, nullptr, stream) != cudaSuccess ||
-        cells_build(view.sph, sph_rad.as<float>(), n, nullptr, 0, kBvhDirRes, kBvhLine, nullptr, 0, nullptr,
-                    dbuf.get(), dbuf.bytes(), &dv, stream) != cudaSuccess) {
+    const uint32_t count = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, pairs / n), n - lists_next);
+    ok = ok && cells_build(view.sph, sph_rad.as<float>(), n, nullptr, 0, kBvhDirRes, kBvhLine, nullptr, 0, nullptr,
+                           dbuf.get(), dbuf.bytes(), &lists_db, stream, lists_next, count) == cudaSuccess;
+    if (!ok) {
         (void)cudaGetLastError();
         clear_error();   // the scene renders on its tree as before
+        lists_lb = LightBufferView{};
+        lists_db = DirBufferView{};
         lbuf.reset();
         dbuf.reset();
         return;
     }
-    view.lb = lv;
-    view.db = dv;
+    lists_next += count;
+    if (lists_next < n) return;
+    view.lb = lists_lb;
+    view.db = lists_db;
 }
 
 uint64_t SceneStore::lists_bytes() const
 {
-    if (!lists_possible(2)) return 0;
+    if (!lists_possible(2) || lists_tried) return 0;
     return lb_bytes(view.n_lights, kBvhLightRes, kBvhLine) + db_bytes(view.n_sph, kBvhDirRes, kBvhLine);
 }
 

@@ -46,19 +46,26 @@ struct SceneStore {
     // than a sixteenth of the device's free memory.
     // Before each render: lists_due counts its paths and says when lists_step
     // has something to do, which is to wait for the renders queued on `work` and
-    // look at the rays they traced, and to build the lists on stream when they pay.
+    // look at the rays they traced, or to build a part of the lists on stream,
+    // of a size that this render's paths pay for (whole: all that is left).
     bool lists_due(uint64_t paths, int32_t bounces);
     atx_status lists_step(uint64_t paths, Budget* budget, cudaStream_t stream, cudaStream_t work);
-    // Whether the lists may still come.
+    // Whether the lists may still come, wholly or in part.
     bool lists_possible(int32_t bounces) const;
-    // granted: the caller has seen to it that lists_bytes() fit its budget.
-    void build_lists(Budget* budget, cudaStream_t stream, bool granted = false);
+    // Builds lists until `pairs` pairs of spheres have been looked at (default:
+    // all of them); they are used once the last are built.  granted: the caller
+    // has seen to it that lists_bytes() fit its budget.
+    void build_lists(Budget* budget, cudaStream_t stream, uint64_t pairs = ~uint64_t(0), bool granted = false);
     // Device bytes of the lists this scene may get (0: none, or it has them).
     uint64_t lists_bytes() const;
     bool lists_on = true;         // renders count towards lists (a server decides when it admits a job)
     uint64_t paths_seen = 0;      // since the upload, until the lists were tried
     uint64_t look_at = 0;         // paths at which the rays are looked at next
-    bool lists_tried = false;     // built or given up
+    double rays_per_path = 0.4;   // after the primary ones, when they were last (before: an open scene's)
+    bool lists_tried = false;     // built, being built or given up
+    uint32_t lists_next = 0;      // the first sphere whose cells are not built yet
+    LightBufferView lists_lb{};   // what view gets when the last are
+    DirBufferView lists_db{};
     uint64_t device_bytes() const
     {
         return sph.bytes() + sph_mat.bytes() + sph_rad.bytes() + mat.bytes() + lights.bytes() + bvh.bytes() +

@@ -100,6 +100,32 @@ def test_lists_in_a_batch_and_after_a_new_scene():
             assert bit_mismatches(got, want[-1]) == 0
 
 
+def _launches(r, spp=2):
+    """Kernels of one render: six through the lists, five on the tree (waves this small)."""
+    before = r.stats()["kernel_launches"]
+    r.render_frames(spp)
+    return r.stats()["kernel_launches"] - before
+
+
+# a build of few and of many parts (4 M pairs of spheres a render of this size): every render in between on the tree
+@pytest.mark.parametrize("kind,n,parts", [("open", 1025, 1), ("open", 4096, 4), ("clump", 8192, 16)])
+@pytest.mark.parametrize("flags", [0, _native.FLAG_OVERLAP_RENDERS])
+def test_lists_are_built_in_parts(kind, n, parts, flags):
+    sc = _scene(kind, n, 5)
+    calls = (1, 2 * n * n // sc.pixels + 1) + (2,) * (parts + 2)
+    want, _ = _render(sc, calls, False, bvh_threshold=1 << 30)
+    used = []
+    with Renderer(flags=flags) as r:
+        r.on_resize(sc.width, sc.height)
+        r.set_scene(sc.spheres, sc.materials, sc.lights)
+        r.set_camera(Camera(sc.fov, sc.near, sc.far, sc.camera_position, sc.camera_direction))
+        r.set_settings(Settings(maxBounces=sc.max_bounces))
+        for spp, w in zip(calls, want):
+            used.append(_launches(r, spp))
+            assert bit_mismatches(r.get_accumulation().reshape(-1, 4), w) == 0
+    assert used[2:] == [5] * (parts - 1) + [6] * 3
+
+
 def test_no_lists_for_rays_that_are_not_traced():
     n = 1100
     sc = _scene("open", n, 4)
