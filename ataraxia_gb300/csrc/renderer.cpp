@@ -70,6 +70,7 @@ atx_status SceneStore::upload(const atx_sphere* s, uint32_t n, const atx_materia
     if (nm) ATX_CUDA(cudaMemcpyAsync(mat.get(), mats.data(), nm * sizeof(DevMaterial), cudaMemcpyHostToDevice, stream));
     if (nl) ATX_CUDA(cudaMemcpyAsync(lights.get(), lts.data(), nl * sizeof(DevLight), cudaMemcpyHostToDevice, stream));
 
+    const bool had_tree = view.use_bvh != 0;
     view = SceneView{};
     view.sph = n ? this->sph.as<float4>() : nullptr;
     view.sph_mat = n ? sph_mat.as<int32_t>() : nullptr;
@@ -105,6 +106,12 @@ atx_status SceneStore::upload(const atx_sphere* s, uint32_t n, const atx_materia
     } else {
         bvh.reset();
         rays.reset();
+    }
+    // the lists of the scene before (up to 6.5 GB) are not held for one that
+    // could not use half of them
+    if (had_tree && lists_bytes() < (lbuf.bytes() + dbuf.bytes()) / 2) {
+        lbuf.reset();
+        dbuf.reset();
     }
     ATX_TRY(build_cells(budget, stream));
     ATX_CUDA(cudaStreamSynchronize(stream));

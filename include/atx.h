@@ -103,7 +103,10 @@ typedef struct atx_config {
     uint32_t bvh_threshold;    /* sphere count at which the LBVH replaces the brute-force tables; 0 = 1025 */
     uint32_t bvh_leaf_size;    /* spheres per BVH leaf; 0 = 8, or what atx_autotune picks */
     uint32_t flags;            /* ATX_FLAG_* */
-    uint64_t hbm_budget_bytes; /* device bytes this renderer may hold; 0 = unlimited */
+    uint64_t hbm_budget_bytes; /* device bytes this renderer may hold; 0 = unlimited (an LBVH scene of up to 8,192
+                                  spheres that goes on being rendered then takes up to a sixteenth of the free
+                                  memory, 0.8 MB a sphere, for tables that replace its tree; with a budget it
+                                  keeps to the tree) */
 } atx_config;
 
 #define ATX_FLAG_NO_GRAPHS 1u       /* launch kernels directly instead of replaying a CUDA graph */

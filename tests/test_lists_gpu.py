@@ -153,3 +153,38 @@ def test_no_lists_for_rays_that_are_not_traced():
         got = r.get_accumulation().reshape(-1, 4)
     want, _ = _render(sc, (frames,) * 12, False, bvh_threshold=1 << 30)
     assert bit_mismatches(got, want[-1]) == 0
+
+
+def test_lists_are_given_back_for_a_smaller_scene():
+    n = 2000
+    big, half, small = _scene("open", n, 4), _scene("open", 1030, 4), _scene("open", 40, 4)
+    frames = 2 * n * n // big.pixels + 1
+    with Renderer(wave_paths=1 << 18) as r:
+        r.on_resize(big.width, big.height)
+        r.set_camera(Camera(big.fov, big.near, big.far, big.camera_position, big.camera_direction))
+        r.set_settings(Settings(maxBounces=big.max_bounces))
+
+        def show(sc):
+            r.set_scene(sc.spheres, sc.materials, sc.lights)
+            r.reset_frame_index()
+            r.render_frames(1)
+            return r.stats()["device_bytes"]
+
+        def go_on():
+            for _ in range(3):
+                r.render_frames(frames)
+            return r.stats()["device_bytes"]
+
+        without = show(big)
+        assert without < n * 300_000
+        assert go_on() > n * 786_432
+        assert show(big) > n * 786_432        # the same scene again: what its lists will need is kept
+        assert go_on() > n * 786_432
+        assert show(half) > n * 786_432       # as for one that needs half of it
+        show(big)
+        go_on()
+        assert show(small) < without + 40 * 400_000   # a table's own buffers
+        show(big)
+        go_on()
+        r.set_scene(half.spheres[:1000], half.materials, half.lights)   # a table, no tree
+        assert r.stats()["device_bytes"] < n * 300_000
