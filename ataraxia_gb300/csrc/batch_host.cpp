@@ -13,16 +13,6 @@ constexpr uint32_t kDefaultLanes = 8;
 constexpr uint32_t kMaxLanes = 64;
 constexpr uint32_t kDefaultLaneWavePaths = 16u << 20;  // 16 Mi paths (about 2.2 GB of path state) per lane
 constexpr uint32_t kDefaultBvhThreshold = 1025;  // LBVH above the direction buffer's 1,024 spheres (64-scene mix: +23% over 512)
-
-// Relative device time of one pass of a scene: paths x (1 + B/2) rays, each
-// N brute-force tests or an LBVH walk, plus a fixed cost per dependent launch
-// (about B + 3 per wave).  Only the order of the estimates matters (LPT).
-double pass_cost(const SceneView& sc, uint64_t paths, int32_t bounces)
-{
-    const double b = std::max(0, bounces);
-    const double per_ray = sc.use_bvh && sc.db.n == 0 ? 100.0 * std::log2((double)sc.n_sph + 2.0) : (double)sc.n_sph + 8.0;
-    return (double)paths * (1.0 + 0.5 * b) * per_ray + 2.0e7 * (b + 3.0);
-}
 }  // namespace
 
 Batch::Batch(const atx_config& cfg) : cfg_(cfg), budget_(cfg.hbm_budget_bytes) {}
@@ -379,7 +369,8 @@ atx_status Batch::run(cudaEvent_t done)
         }
         const uint64_t want = (p + tuning_.lane_wave_paths - 1) / tuning_.lane_wave_paths;
         const uint32_t n = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({want, max_lanes, px}));
-        const double c = pass_cost(s->scene.view, p, s->settings.max_bounces) / n;
+        const SceneView& v = s->scene.view;
+        const double c = pass_cost(v.n_sph, v.use_bvh && v.db.n == 0, p, s->settings.max_bounces) / n;
         for (uint32_t k = 0; k < n; ++k) parts.push_back({i, c, px * k / n, px * (k + 1) / n});
     }
     ++st_.passes;

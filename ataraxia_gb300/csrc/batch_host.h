@@ -20,6 +20,7 @@
 // lane), so passes overlap instead of meeting at a barrier.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <memory>
 #include <vector>
@@ -29,6 +30,22 @@
 #include "renderer.h"
 
 namespace atx {
+
+// Device time of one pass of a scene on one lane, estimated in picoseconds:
+// paths x (1 + B/2) rays, each through the tables (brute-force scenes, LBVH
+// scenes with cell lists) or a walk of the tree, plus the chain of its launches.
+// Fitted to open scenes, 16 samples of 1280x720 pixels, 8 bounces, measured /
+// estimated: tables of 9, 256 and 1,000 spheres 1.02 / 1.22, 2.1 / 1.8 and 3.8 /
+// 3.7 ps, lists of 4,096 and 8,000 11.3 / 11.4 and 20.0 / 21.2, trees of 1,025,
+// 4,096, 8,000 and 40,000 19.6 / 19.9, 51 / 49, 78 / 76 and 217 / 216; a pass of
+// 64x64 pixels 12 to 53 us.  Only the order of the estimates matters (longest
+// first onto the least-loaded lane).
+inline double pass_cost(uint32_t n_spheres, bool walks, uint64_t paths, int32_t bounces)
+{
+    const double n = n_spheres, b = bounces > 0 ? bounces : 0;
+    const double per_ray = walks ? 0.22 * std::pow(n, 0.65) : 1.2 + 0.0025 * n;
+    return (double)paths * (1.0 + 0.5 * b) * per_ray + 3.5e7;
+}
 
 class Batch {
 public:
