@@ -932,7 +932,8 @@ namespace {
 
 // Tuned settings kept per process, keyed by the GPU (SM count and compute
 // capability) and a bucket of the workload: log2 of the sphere count, the
-// nearest-hit structure (LBVH, or brute force with light buffer or without),
+// nearest-hit structure (LBVH with cell lists or without, brute force with
+// light buffer or without),
 // log2 of the paths per launch and the bounce depth.
 struct TuneKey {
     int sms, cc;
@@ -1050,8 +1051,15 @@ atx_status Renderer::autotune(uint32_t spp, uint32_t passes, bool use_cache, atx
     ATX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg_.device));
     ATX_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, cfg_.device));
     ATX_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, cfg_.device));
+    // the trials are renders of one scene: lists it would get on the way come first
+    // (they run other kernels than the tree, so the settings are kept apart)
+    if (scene_.lists_possible(settings_.max_bounces)) {
+        ATX_TRY(join());
+        scene_.build_lists(&budget_, stream_);
+        stream_dirty_ = true;
+    }
     const SceneView& sv = scene_.view;
-    const int kind = sv.use_bvh ? 2 : (sv.lb.n_lights ? 1 : 0);
+    const int kind = sv.use_bvh ? (sv.db.n ? 3 : 2) : (sv.lb.n_lights ? 1 : 0);
     const TuneKey key{sms, 10 * major + minor, log2_bucket(sv.n_sph + 1ull), kind,
                       log2_bucket((uint64_t)width_ * height_ * spp), settings_.max_bounces};
     if (use_cache) {
@@ -1072,12 +1080,6 @@ atx_status Renderer::autotune(uint32_t spp, uint32_t passes, bool use_cache, atx
             frame_ = 1;
             return tuning(out);
         }
-    }
-    // the trials are renders of one scene: lists it would get on the way come first
-    if (scene_.lists_possible(settings_.max_bounces)) {
-        ATX_TRY(join());
-        scene_.build_lists(&budget_, stream_);
-        stream_dirty_ = true;
     }
     // coordinate descent from the defaults: leaf size, then lanes, path state,
     // block size and the wave's tile shape, each keeping the best so far

@@ -100,3 +100,24 @@ def test_cell_resolution_outside_its_range_is_rejected(res):
         with pytest.raises(AtxError):
             r.set_tuning(cell_res=res)
         assert r.tuning()["cell_res"] == 32
+
+
+def test_settings_for_lists_and_for_the_tree_are_kept_apart(po):
+    sc = _scene("lbvh").with_resolution(320, 180)
+    sc.spheres, sc.max_bounces = sc.spheres[:1100].copy(), 3
+
+    def tuned(budget):
+        with Renderer(hbm_budget_bytes=budget) as r:   # with a budget the scene keeps to its tree
+            r.on_resize(sc.width, sc.height)
+            r.set_scene(sc.spheres, sc.materials, sc.lights)
+            view = po.view_for(sc)
+            r.set_camera_matrices(np.array(view.inv_view), np.array(view.inv_proj), sc.camera_position)
+            r.set_settings(Settings(accumulation=True, skyLight=False, maxBounces=sc.max_bounces))
+            return r.autotune(2, passes=1)["from_cache"], r.stats()["device_bytes"]
+
+    budget = 8 << 30
+    first, tree = tuned(budget)
+    other, lists = tuned(0)
+    assert lists > tree + 1100 * 700_000
+    assert (first, other) == (0, 0)
+    assert tuned(0)[0] == 1 and tuned(budget)[0] == 1
