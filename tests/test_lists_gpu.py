@@ -188,3 +188,22 @@ def test_lists_are_given_back_for_a_smaller_scene():
         go_on()
         r.set_scene(half.spheres[:1000], half.materials, half.lights)   # a table, no tree
         assert r.stats()["device_bytes"] < n * 300_000
+
+
+def test_lists_of_more_spheres_in_a_face_than_a_block_keeps():
+    from test_cells_gpu import slab
+
+    n = 4000
+    sc = slab(n)
+    calls = (1, 2 * n * n // sc.pixels + 1) + (2,) * 6
+    want, _ = _render(sc, calls, True, bvh_threshold=1 << 30)
+    with Renderer() as r:
+        r.on_resize(sc.width, sc.height)
+        r.set_scene(sc.spheres, sc.materials, sc.lights)
+        r.set_camera(Camera(sc.fov, sc.near, sc.far, sc.camera_position, sc.camera_direction))
+        r.set_settings(Settings(skyLight=True, maxBounces=sc.max_bounces))
+        used = []
+        for spp, w in zip(calls, want):
+            used.append(_launches(r, spp))
+            assert bit_mismatches(r.get_accumulation().reshape(-1, 4), w) == 0
+    assert used[-1] == 6
