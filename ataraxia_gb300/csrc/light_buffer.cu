@@ -20,8 +20,13 @@
 // the lookup finds lists the sphere: a cell lists every sphere whose cap,
 // widened by 1e-4 rad for the lookup's rounding, meets the cell's bounding
 // cone.  A sphere whose centre lies within R' + m of the light (the segment
-// could end inside it) is listed in every cell.  The direction buffer's lists
-// are built the same way (its own note below).
+// could end inside it) is listed in every cell.  Spheres whose caps miss the
+// bounding cone of the cell's whole face, widened by 8e-3 rad, are left out
+// beforehand: the directions of a cell lie in that cone, so a cap that holds
+// one of them, give or take the lookup's 1e-4 rad, meets it (a cap that meets
+// only the part of a cell's bounding cone that sticks out of the face holds
+// none).  The direction buffer's lists are built the same way (its own note
+// below).
 #include "light_buffer.h"
 
 namespace atx {

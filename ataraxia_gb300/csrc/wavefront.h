@@ -96,8 +96,12 @@ constexpr uint32_t kCellResMin = 8;
 constexpr uint32_t kCellResMax = 32;
 constexpr uint32_t kCellResDefault = 32;   // a renderer's and a batch's resident scenes
 constexpr uint32_t kCellResJobs = 16;      // the server's jobs (tables built per job)
-// Up to this many spheres the lists are about one sphere already at 16, and
-// finer cells only make the tables larger (the 9-sphere scene: -1% at 32).
+// Up to this many spheres finer cells only make the tables larger: 48 spread
+// spheres list 1.5 an extension ray and 2 a shadow ray at 16 already.  A sphere
+// of the scene's size leaves little to cull at any resolution, since the margins
+// grow with the scene: 8 spheres on a ground of radius 1000 list 7.5 to 8.5 of 9
+// after the first bounce (all 9 for rays that leave the ground), 4 to 8 a shadow
+// ray (-1% at 32).
 constexpr uint32_t kCellResFewSpheres = 64;
 __host__ __device__ constexpr uint32_t default_cell_res(uint32_t n_spheres)
 {
@@ -125,7 +129,7 @@ struct LightBufferView {
 // hit, so its nearest hit tests the spheres of one cell.
 constexpr uint32_t kDbMaxSpheres = 1024;   // 393 KB of cells per sphere at res 32
 // LBVH scenes up to this many spheres get both buffers too, once they have
-// traced enough paths to pay for the build (SceneStore::lists_due), at these
+// traced enough rays to pay for the build (SceneStore::lists_step), at these
 // resolutions and with lines twice as long (63 spheres).  A lookup and a few
 // spheres replace a walk that runs 5 to 9 of a warp's 32 lanes: 16 samples of
 // 1280x720 pixels over 4,096 spheres 3.05 -> 0.56 ms (0.66 at 24 cells, 1.23 with
